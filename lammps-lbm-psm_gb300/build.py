@@ -36,6 +36,7 @@ def nvcc() -> str:
 
 def _deps(unit: str) -> list[str]:
     return [os.path.join(CSRC, unit + ".cu"), os.path.join(CSRC, "lbmpsm_internal.cuh"),
+            os.path.join(CSRC, "solid_fraction.cuh"),
             os.path.join(ROOT, "include", "lbmpsm.h")]
 
 

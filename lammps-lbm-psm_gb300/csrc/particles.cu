@@ -15,8 +15,8 @@
 //   4. cell_sort  : sort each list ascending (restores image order)
 //   5. node_apply : per node, walk its cell's list and apply the 4-way update
 // The solid fraction counts the reference's 10^d sub-cell centres; each
-// comparison is decided in FP32 when it is far from the threshold (a margin
-// 250x the worst FP32 error) and otherwise evaluated with the reference's
+// comparison is decided in FP32 when it is far from the threshold (proven
+// margins, solid_fraction.cuh) and otherwise evaluated with the reference's
 // FP64 expression, so the count is the reference's count.
 //
 // Reduce (replaces calculateHydrodynamicInteractions,
@@ -24,6 +24,7 @@
 // the node forces of its tag over the box clamped to interior nodes, with a
 // fixed-order warp-shuffle and block reduction (deterministic run to run).
 #include "lbmpsm_internal.cuh"
+#include "solid_fraction.cuh"
 
 namespace lbmpsm {
 
@@ -143,12 +144,7 @@ __global__ void img_prep_kernel(MapParams p) {
     im.rSqf = (float)im.rSq;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      // xl = xi + xfrac exactly (the fractional part of a double is exact)
-      const double xl = im.xl[d];
-      const bool small = fabs(xl) < 1.0e9;
-      const double fl = small ? floor(xl) : 0.0;
-      im.xi[d] = (int)fl;
-      im.xf[d] = (float)(xl - fl);
+      split_centre(im.xl[d], im.xi[d], im.xf[d]);
     }
     // the node velocity reduces to uT + 0.0 bit for bit when every omega
     // component is +0.0 and no uT component is -0.0 (signed-zero arithmetic)
@@ -366,38 +362,6 @@ __global__ void cell_sort_kernel(MapParams p, int ncells) {
     }
 }
 
-// Early-out part of calcSolidFraction for one node, decided in FP32 with a
-// proven margin, else in FP64 with the reference's expressions.  Returns a
-// code (0 or SF_ONE) or -1 for a shell node whose sub-cells must be counted.
-//
-// Offsets dx = (double)h - xl are formed as (h - xi) - xfrac with xl = xi + xfrac
-// split exactly, so |dxf - dx| <= u(|dx| + 1), u = 2^-24, and the FP32 squared
-// distance obeys |d32 - dist| <= u(5 dist + 2 sum|d|).  The margin m is 16x that.
-static __device__ __forceinline__ int classify_node(int hi, int hj, int hk, const Img& im,
-                                                    float& dxf, float& dyf, float& dzf) {
-  const float u = 5.9604644775390625e-08f;  // 2^-24
-  dxf = small_int_to_float(hi - im.xi[0]) - im.xf[0];
-  dyf = small_int_to_float(hj - im.xi[1]) - im.xf[1];
-  dzf = small_int_to_float(hk - im.xi[2]) - im.xf[2];
-  const float d32 = dxf * dxf + dyf * dyf + dzf * dzf;
-  const float ad = fabsf(dxf) + fabsf(dyf) + fabsf(dzf);
-  const float m = 16.0f * u * (5.0f * d32 + 2.0f * ad + 1.0f + im.rP2f);
-  if (d32 > im.rP2f + m) return 0;
-  const bool nearP = d32 >= im.rP2f - m;
-  const bool nearM = d32 >= im.rM2f - m && d32 <= im.rM2f + m;
-  if (nearP || nearM) {
-    const double dx = (double)hi - im.xl[0];
-    const double dy = (double)hj - im.xl[1];
-    const double dz = (double)hk - im.xl[2];
-    const double dist = dx * dx + dy * dy + dz * dz;
-    if (dist > im.rP2) return 0;
-    if (dist < im.rM2) return SF_ONE;
-    return -1;
-  }
-  if (d32 < im.rM2f) return SF_ONE;  // below rM^2 - m: inside for certain
-  return -1;
-}
-
 // A shell node (between the early-out radii) whose sub-cells all lie on one
 // side of the surface: the count calcSolidFraction's loop would give
 // (src/LBM_PSM_exchangeParticleData.cpp:151-165), 10^dim or 0, else -1.
@@ -425,11 +389,6 @@ static __device__ __forceinline__ int corner_count(int dim, float dxf, float dyf
 
 constexpr int SFC_THREADS = 64;   // classification: one block per image
 constexpr int SFS_THREADS = 128;  // shell counting: persistent warps
-constexpr int SFS_BUF = 352;      // per-warp buffer of crossing rows (>= 32 + 32*10)
-
-static __device__ __forceinline__ float sub_offset(int k) {
-  return -0.45f + 0.1f * small_int_to_float(k);  // within 1.7u of the reference's delta_k
-}
 
 // Phase 1 of the map, one block per image.  The box's codes are first set
 // to 0 with coalesced stores; then only the nodes of each x-row that may
@@ -534,302 +493,24 @@ __global__ void __launch_bounds__(SFC_THREADS) sf_classify_kernel(MapParams p) {
   if (qn) flush();
 }
 
-// Exact double of a small non-negative integer without the conversion unit.
-static __device__ __forceinline__ double small_int_to_double(int k) {
-  return __hiloint2double(0x43300000, k) - 4503599627370496.0;  // 2^52 + k - 2^52
-}
-
-// One row of sub-cells whose FP32 decision is not certain: the row fixes
-// sub-cell index ia on axis pa and ib on axis pb and runs over the 10
-// indices c of the remaining axis.  Sub-cells whose FP32 c-term lies below
-// the band count as inside, above it as outside, and the ones inside the
-// band are decided with the reference's FP64 expressions
-// (src/LBM_PSM_exchangeParticleData.cpp:144-168).  Kept out of line so that
-// the rare branch calling it is not predicated into every row.
-static __device__ __noinline__ int exact_row_count(const Img& im, int hx, int hy, int hz, int pa,
-                                                   int pb, int ia, int ib, float dc, float tlo,
-                                                   float thi) {
-  const double sliceWidth = 1.0 / ((double)10);
-  const double rSq = im.r * im.r;
-  const double D[3] = {small_int_to_double(hx) - im.xl[0], small_int_to_double(hy) - im.xl[1],
-                       small_int_to_double(hz) - im.xl[2]};
-  int n = 0;
-#pragma unroll
-  for (int c = 0; c < 10; ++c) {
-    const float t = dc + (float)(-0.5 + ((double)c + 0.5) * 0.1);
-    const float sc = t * t;
-    if (sc < tlo) {
-      ++n;
-    } else if (sc <= thi) {
-      const int i0 = pa == 0 ? ia : (pb == 0 ? ib : c);
-      const int i1 = pa == 1 ? ia : (pb == 1 ? ib : c);
-      const int i2 = pa == 2 ? ia : (pb == 2 ? ib : c);
-      const double t0 = D[0] + (-0.5 + (small_int_to_double(i0) + 0.5) * sliceWidth);
-      const double t1 = D[1] + (-0.5 + (small_int_to_double(i1) + 0.5) * sliceWidth);
-      const double t2 = D[2] + (-0.5 + (small_int_to_double(i2) + 0.5) * sliceWidth);
-      const double ax = t0 * t0, ay = t1 * t1, az = t2 * t2;
-      if (ax + ay + az < rSq) ++n;
-    }
-  }
-  return n;
-}
-
-// The same for a whole 2-D node (10 x 10 sub-cells).
-static __device__ __noinline__ int exact_count_2d(const Img& im, int hx, int hy) {
-  const double sliceWidth = 1.0 / ((double)10);
-  const double rSq = im.r * im.r;
-  const double D0 = (double)hx - im.xl[0], D1 = (double)hy - im.xl[1];
-  int n = 0;
-  for (int a = 0; a < 10; ++a) {
-    const double ta = D0 + (-0.5 + ((double)a + 0.5) * sliceWidth);
-    const double ax = ta * ta;
-    for (int b = 0; b < 10; ++b) {
-      const double tb = D1 + (-0.5 + ((double)b + 0.5) * sliceWidth);
-      if (ax + tb * tb < rSq) ++n;
-    }
-  }
-  return n;
-}
-
-// Phase 2: sub-cell counts of the shell nodes, one node per lane, the list
-// walked by a persistent grid in warp-sized chunks.
-//
-// 3-D: with the axes ordered so that the inner axis c has the smallest
-// |offset| (its rows run most nearly along the sphere surface, so fewest of
-// them cross it), a node's sub-cells are 10 slabs a of 100 rows (a, b).  A
-// row whose 10 sub-cell sums are all below r^2 - M counts 10, one whose sums
-// are all above r^2 + M counts 0 (M bounds the FP32 error, 16x the worst
-// case); a row in between crosses the surface.  Each lane first tests its
-// node's slabs as wholes: a slab whose largest row sum (its a-term plus the
-// largest b-term) passes the inside test counts 100, one whose smallest
-// fails the outside test counts 0 -- exactly what its rows would give, the
-// FP32 sums being monotone in each term.  The other slabs go to a per-warp
-// queue, taken one slab per lane: the slab's rows are tested and its
-// crossing rows pushed into a per-warp buffer that is drained 32 rows at a
-// time, one row per lane: the count is the rank of r^2 - M - s_ab among the
-// node's 10 sorted c-terms, and a c-term within the margin band makes the
-// row ambiguous, in which case that row alone is recounted exactly in FP64.
-// 2-D: 100 sub-cells per node, counted in FP32 with the same margin; a node
-// with any ambiguous sub-cell is recounted exactly.
+// Phase 2: sub-cell counts of the shell nodes (shell_count, the rule and its
+// margins there), one node per lane, the list walked by a persistent grid in
+// warp-sized chunks.  Every lane walks the same 100 rows without branches or
+// shared memory (suspension of 2260 images in 256^3: 60 us; sorting each
+// node's terms and compacting its crossing rows across the warp took 135).
 __global__ void __launch_bounds__(SFS_THREADS, 8) sf_shell_kernel(MapParams p) {
-  constexpr int NW = SFS_THREADS / 32;
-  __shared__ float s_sorted[NW][32][17];  // 10 sorted c-terms + padding (odd stride)
-  __shared__ float s_lo[NW][32];
-  __shared__ float s_hi[NW][32];
-  __shared__ int s_cnt[NW][32];
-  __shared__ int s_ent[NW][32];   // shell-list entry of each lane's node
-  __shared__ int s_perm[NW][32];  // its axis order: pa | pb << 2
-  __shared__ float s_dc[NW][32];  // its inner-axis offset
-  __shared__ float buf_s[NW][SFS_BUF];
-  __shared__ unsigned short buf_o[NW][SFS_BUF];   // owner lane | a << 5 | b << 9
-  __shared__ unsigned short q_slab[NW][32 * 10];  // partial slabs: owner lane | a << 5
-  __shared__ float s_da[NW][32], s_db[NW][32], s_lin[NW][32], s_hout[NW][32];
   const unsigned long long tot = p.pair_total[2];
   const int total = (int)min(tot, (unsigned long long)p.shell_cap);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gw = blockIdx.x * NW + warp, nw = gridDim.x * NW;
-  const float u = 5.9604644775390625e-08f;  // 2^-24
-  const Geom& g = p.g;
-#pragma unroll
-  for (int k = 10; k < 16; ++k) s_sorted[warp][lane][k] = 3.0e38f;
-  for (int base = gw * 32; base < total; base += nw * 32) {
-    const int e = base + lane;
-    const bool valid = e < total;
-    const int4 ent = p.shell[valid ? e : base];
+  const int stride = (int)(gridDim.x * SFS_THREADS);
+  for (int e = (int)(blockIdx.x * SFS_THREADS + threadIdx.x); e < total; e += stride) {
+    const int4 ent = p.shell[e];
     const Img& im = p.img[ent.x];
-    const int hx = ent.z & 0xFFFF, hy = ent.z >> 16, hz = ent.w;
+    const int hx = ent.z & 0xFFFF, hy = (int)((unsigned)ent.z >> 16), hz = ent.w;
     const float dxf = small_int_to_float(hx - im.xi[0]) - im.xf[0];
     const float dyf = small_int_to_float(hy - im.xi[1]) - im.xf[1];
     const float dzf = small_int_to_float(hz - im.xi[2]) - im.xf[2];
-    const float rSqf = im.rSqf;
-    int n = 0;
-    if (g.dim == 2) {
-      const float Ea = fabsf(dxf) + 2.0f, Eb = fabsf(dyf) + 2.0f;
-      const float M = 16.0f * u * (Ea * Ea + Eb * Eb + rSqf);
-      const float lo = rSqf - M, hi = rSqf + M;
-      int amb = 0;
-      for (int a = 0; a < 10; ++a) {
-        const float ta = dxf + sub_offset(a);
-        const float sa = ta * ta;
-#pragma unroll
-        for (int b = 0; b < 10; ++b) {
-          const float tb = dyf + (float)(-0.5 + ((double)b + 0.5) * 0.1);
-          const float t = sa + tb * tb;
-          n += (t < lo);
-          amb += (t >= lo) & (t <= hi);
-        }
-      }
-      if (valid && amb) n = exact_count_2d(im, hx, hy);
-    } else {
-      // axis order: inner c along the smallest |offset| (its rows run most
-      // nearly along the surface, so fewest cross it), outer a along the
-      // largest (the surface crosses the node nearly perpendicular to it, so
-      // fewest slabs are partial), middle b the other
-      float da = dxf, db = dyf, dc = dzf;
-      int pa = 0, pb = 1;
-      {
-        const float ax = fabsf(dxf), ay = fabsf(dyf), az = fabsf(dzf);
-        if (ax <= ay && ax <= az) {
-          da = dyf; db = dzf; dc = dxf; pa = 1; pb = 2;
-        } else if (ay <= ax && ay <= az) {
-          da = dxf; db = dzf; dc = dyf; pa = 0; pb = 2;
-        }
-        if (fabsf(db) > fabsf(da)) {  // outer and middle swap: sums and margins are symmetric
-          const float t = da; da = db; db = t;
-          const int q = pa; pa = pb; pb = q;
-        }
-      }
-      const float Ea = fabsf(da) + 2.0f, Eb = fabsf(db) + 2.0f, Ec = fabsf(dc) + 2.0f;
-      const float M = 16.0f * u * (Ea * Ea + Eb * Eb + Ec * Ec + rSqf);
-      const float lo = rSqf - M, hi = rSqf + M;
-      // the 10 c-terms, sorted (odd-even transposition)
-      float sc[10];
-#pragma unroll
-      for (int c = 0; c < 10; ++c) {
-        const float t = dc + (float)(-0.5 + ((double)c + 0.5) * 0.1);
-        sc[c] = t * t;
-      }
-#pragma unroll
-      for (int r = 0; r < 10; ++r) {
-#pragma unroll
-        for (int c = r & 1; c + 1 < 10; c += 2) {
-          const float x = fminf(sc[c], sc[c + 1]), y = fmaxf(sc[c], sc[c + 1]);
-          sc[c] = x;
-          sc[c + 1] = y;
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 10; ++c) s_sorted[warp][lane][c] = sc[c];
-      s_lo[warp][lane] = lo;
-      s_hi[warp][lane] = hi;
-      s_cnt[warp][lane] = 0;
-      const float lo_in = lo - sc[9];   // row wholly inside: s_ab + max c-term < lo
-      const float hi_out = hi - sc[0];  // row wholly outside: s_ab + min c-term > hi
-      float sb_min = 3.0e38f, sb_max = 0.0f;
-#pragma unroll
-      for (int b = 0; b < 10; ++b) {
-        const float t = db + sub_offset(b);
-        const float v = t * t;
-        sb_min = fminf(sb_min, v);
-        sb_max = fmaxf(sb_max, v);
-      }
-      s_ent[warp][lane] = valid ? e : base;
-      s_perm[warp][lane] = pa | (pb << 2);
-      s_dc[warp][lane] = dc;
-      s_da[warp][lane] = da;
-      s_db[warp][lane] = db;
-      s_lin[warp][lane] = lo_in;
-      s_hout[warp][lane] = hi_out;
-      // whole slabs: inside (100), outside (0), or partial (queued)
-      unsigned pm = 0;
-#pragma unroll
-      for (int a = 0; a < 10; ++a) {
-        const float ta = da + sub_offset(a);
-        const float sa = ta * ta;
-        const bool in = sa + sb_max < lo_in;
-        const bool out = sa + sb_min > hi_out;
-        n += in ? 100 : 0;
-        pm |= (!in && !out) ? (1u << a) : 0u;
-      }
-      if (!valid) pm = 0;
-      int nslab;
-      {
-        const int cnt = __popc(pm);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        int pos = incl - cnt;
-        while (pm) {
-          const int a = __ffs(pm) - 1;
-          pm &= pm - 1u;
-          q_slab[warp][pos++] = (unsigned short)(lane | (a << 5));
-        }
-        nslab = __shfl_sync(0xffffffffu, incl, 31);
-      }
-      __syncwarp();
-      // count of one buffered crossing row, added to its owner lane
-      auto drain_row = [&](int k) {
-        const float sv = buf_s[warp][k];
-        const int o = buf_o[warp][k];
-        const int ow = o & 31;
-        const float tlo = s_lo[warp][ow] - sv, thi = s_hi[warp][ow] - sv;
-        const float* srt = s_sorted[warp][ow];
-        int r = 0;  // number of c-terms below tlo (entries 10..15 are +huge)
-        if (srt[r + 7] < tlo) r += 8;
-        if (srt[r + 3] < tlo) r += 4;
-        if (srt[r + 1] < tlo) r += 2;
-        if (srt[r] < tlo) r += 1;
-        int rc = r;
-        if (srt[r] <= thi) {  // a c-term inside the margin band: decide it exactly
-          const int4 oe = p.shell[s_ent[warp][ow]];
-          const int pp = s_perm[warp][ow];
-          rc = exact_row_count(p.img[oe.x], oe.z & 0xFFFF, oe.z >> 16, oe.w, pp & 3, pp >> 2,
-                               (o >> 5) & 15, (o >> 9) & 15, s_dc[warp][ow], tlo, thi);
-        }
-        if (rc) atomicAdd(&s_cnt[warp][ow], rc);
-      };
-      int wtotal = 0;  // rows in the warp buffer (warp-uniform)
-      for (int k0 = 0; k0 < nslab; k0 += 32) {
-        // one partial slab per lane: its rows, the crossing ones buffered
-        unsigned cm = 0;
-        int ow = 0, a = 0;
-        float sa = 0.0f;
-        if (k0 + lane < nslab) {
-          const int q = q_slab[warp][k0 + lane];
-          ow = q & 31;
-          a = q >> 5;
-          const float ta = s_da[warp][ow] + sub_offset(a);
-          sa = ta * ta;
-          const float dbo = s_db[warp][ow], lin = s_lin[warp][ow], hout = s_hout[warp][ow];
-          int in_rows = 0;
-#pragma unroll
-          for (int b = 0; b < 10; ++b) {
-            const float tb = dbo + sub_offset(b);
-            const float sv = sa + tb * tb;
-            const bool inside = sv < lin;
-            in_rows += inside ? 10 : 0;
-            cm |= (!inside && sv <= hout) ? (1u << b) : 0u;
-          }
-          if (in_rows) atomicAdd(&s_cnt[warp][ow], in_rows);
-        }
-        // append the crossing rows to the warp buffer
-        const int cnt = __popc(cm);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        int pos = wtotal + incl - cnt;
-        if (cm) {
-          const float dbo = s_db[warp][ow];
-          while (cm) {
-            const int b = __ffs(cm) - 1;
-            cm &= cm - 1u;
-            const float tb = dbo + sub_offset(b);
-            buf_s[warp][pos] = sa + tb * tb;
-            buf_o[warp][pos] = (unsigned short)(ow | (a << 5) | (b << 9));
-            ++pos;
-          }
-        }
-        wtotal += __shfl_sync(0xffffffffu, incl, 31);
-        __syncwarp();
-        // drain 32 rows at a time, one per lane
-        while (wtotal >= 32) {
-          drain_row(wtotal - 32 + lane);
-          wtotal -= 32;
-          __syncwarp();
-        }
-      }
-      if (lane < wtotal) drain_row(lane);
-      __syncwarp();
-      n += s_cnt[warp][lane];
-      __syncwarp();
-    }
-    if (valid) p.sfcode[im.sf_off + ent.y] = (unsigned short)n;
+    p.sfcode[im.sf_off + ent.y] =
+        (unsigned short)shell_count(p.g.dim, im, hx, hy, hz, dxf, dyf, dzf);
   }
 }
 
