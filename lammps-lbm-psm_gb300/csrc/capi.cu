@@ -1835,6 +1835,8 @@ int lbmpsm_adjoint_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   CUDA_TRY(h, sc.get(&sums, sizeof(double) * ADJ_PART));
   CUDA_TRY(h, sc.get(&drag, sizeof(double) * (size_t)T));
   CUDA_TRY(h, sc.get(&gx, sizeof(double) * 3 * (size_t)std::max(n, 1)));
+  double* gpart = nullptr;
+  CUDA_TRY(h, sc.get(&gpart, sizeof(double) * 3 * ADJ_CEN_PARTS * (size_t)std::max(n, 1)));
   CUDA_TRY(h, cudaMemsetAsync(part, 0, sizeof(double) * ADJ_PART * (size_t)nb, h->stream));
   CUDA_TRY(h, cudaMemsetAsync(drag, 0, sizeof(double) * (size_t)T, h->stream));
   CUDA_TRY(h, cudaMemsetAsync(gx, 0, sizeof(double) * 3 * (size_t)std::max(n, 1), h->stream));
@@ -1887,6 +1889,7 @@ int lbmpsm_adjoint_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   }
   AdjCentre c = adj_centre(h, an, n, centre_step);
   c.out = gx;
+  c.part = gpart;
   CUDA_TRY(h, launch_adj_centre(c, h->stream));
   CUDA_TRY(h, launch_adj_sum(part, nb, sums, h->stream));
   std::vector<double> hd((size_t)T), hs(ADJ_PART), hx(3 * (size_t)std::max(n, 1));

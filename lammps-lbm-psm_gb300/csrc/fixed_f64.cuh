@@ -1,0 +1,157 @@
+// fixed_f64.cuh -- IEEE double additions of the collide step on the integer
+// units, bit for bit.
+//
+// This GPU issues 1.68 FP64 operations per clock and multiprocessor against
+// about 100 integer ones, and both at once, so an addition whose rounding
+// position is known can be had for a dozen integer instructions beside the
+// FP64 pipe.  Near equilibrium it is known: populations, their sums and the
+// factors 1 + 3 e.u + ... of the equilibria keep to one or two binades.  The
+// values are held as 64-bit integers in units of 2^-60 (populations and
+// sums) or 2^-62 (the factors); each result is rounded to 53 significant bits,
+// ties to even, as the IEEE addition it stands for.  Every function states
+// the range it needs; the caller checks the ranges (populations in
+// [2^-6, 1), velocity components below 1/16 and the sums below) and takes the
+// FP64 expressions otherwise.
+//
+// Host compilable: the functions are compared with IEEE arithmetic on the CPU.
+#pragma once
+
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define LBMPSM_HD __host__ __device__ __forceinline__
+#else
+#define LBMPSM_HD inline
+#endif
+
+namespace lbmpsm {
+namespace fx {
+
+typedef unsigned long long u64;
+typedef long long i64;
+
+LBMPSM_HD u64 bits_of(double x) {
+#ifdef __CUDA_ARCH__
+  return (u64)__double_as_longlong(x);
+#else
+  u64 b;
+  memcpy(&b, &x, 8);
+  return b;
+#endif
+}
+LBMPSM_HD double of_bits(u64 b) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((i64)b);
+#else
+  double x;
+  memcpy(&x, &b, 8);
+  return x;
+#endif
+}
+LBMPSM_HD int clz64(u64 x) {  // x != 0
+#ifdef __CUDA_ARCH__
+  return __clzll((i64)x);
+#else
+  return __builtin_clzll(x);
+#endif
+}
+
+// f in units of 2^-60; f in [2^-6, 1), else bad becomes non-zero.  The result
+// is a multiple of 4.
+LBMPSM_HD u64 to60(double f, unsigned& bad) {
+  const u64 b = bits_of(f);
+  const unsigned hi = (unsigned)(b >> 32);
+  const unsigned s = (hi >> 20) - (1023u - 6u);  // 0..5; sign, small, large, inf, NaN: beyond
+  bad |= s > 5u ? 1u : 0u;
+  const u64 m = ((u64)((hi & 0xFFFFFu) | 0x100000u) << 32) | (b & 0xFFFFFFFFull);
+  return m << ((s + 2u) & 7u);
+}
+
+// t rounded to a multiple of 2^sh, ties to even (t >= 0)
+LBMPSM_HD u64 rne(u64 t, int sh) {
+  return (t + ((1ull << (sh - 1)) - 1ull) + ((t >> sh) & 1ull)) & ~((1ull << sh) - 1ull);
+}
+
+// t >= 0 in units of 2^-60, rounded to 53 bits: t in [2^(58+k0), 2^(60+k0))
+// where k0 = 0 (t in [1/4, 1)) or 1 (t in [1/2, 2))
+LBMPSM_HD u64 rne53_of2(u64 t, int k0) {
+  const unsigned c = (unsigned)(t >> (59 + k0)) & 1u;
+  const int sh = 6 + k0 + (int)c;
+  const u64 half = 32ull << (k0 + (int)c);
+  return (t + (half - 1ull) + ((t >> sh) & 1ull)) & ~(2ull * half - 1ull);
+}
+
+// t (a multiple of 4, |t| < 2^57, units of 2^-60) rounded to 53 bits
+LBMPSM_HD i64 rne53_signed(i64 t) {
+  const unsigned a = (unsigned)(((u64)t >> 32) ^ (u64)(i64)(t >> 63));  // high word of |t| (or |t| - 1)
+  const unsigned m = a >= (1u << 24) ? 15u : (a >= (1u << 23) ? 7u : 0u);
+  const int sh = a >= (1u << 24) ? 4 : 3;
+  const unsigned low = (unsigned)t;
+  const u64 inc = (u64)((m >> 1) + ((low >> sh) & 1u & m));
+  return (i64)(((u64)t + inc) & ~(u64)m);
+}
+
+// the double t * 2^-60 (t with at most 53 significant bits)
+LBMPSM_HD double from60(i64 t) {
+  const u64 sg = (u64)t & 0x8000000000000000ull;
+  const u64 a = t < 0 ? (u64)0 - (u64)t : (u64)t;
+  if (a == 0) return 0.0;
+  const int lz = clz64(a);
+  const u64 m = (a << lz) >> 11;  // 53 bits, the leading one at bit 52
+  return of_bits(sg | (m + ((u64)(1025 - lz) << 52)));
+}
+
+// the double t * 2^-60 for a 53-bit t in [1/2, 2)
+LBMPSM_HD double from60_near1(u64 t) {
+  const unsigned c = (unsigned)(t >> 60);
+  return of_bits((t >> (7 + c)) + ((u64)(1021u + c) << 52));
+}
+
+// |x| in units of 2^-62, |x| < 1/2: bits below the unit are kept as a set
+// lowest bit ("sticky"), which rounds like them at any position above bit 1
+LBMPSM_HD u64 align62(double x) {
+  const u64 b = bits_of(x);
+  const unsigned e = (unsigned)(b >> 52) & 0x7FFu;
+  const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull)) << 8;
+  const unsigned r0 = 1021u - e;
+  const unsigned r = r0 < 63u ? r0 : 63u;
+  const u64 a = m >> r;
+  return (a << r) != m ? (a | 1ull) : a;
+}
+
+constexpr u64 ONE62 = 1ull << 62;
+
+// s >= 0 in units of 2^-62 rounded to 53 bits: s in [1/2, 2)
+LBMPSM_HD u64 rne53_62(u64 s) {
+  const unsigned c = (unsigned)(s >> 62);
+  const int sh = 9 + (int)c;
+  const u64 half = 256ull << c;
+  return (s + (half - 1ull) + ((s >> sh) & 1ull)) & ~(2ull * half - 1ull);
+}
+
+// the double s * 2^-62 for a 53-bit s in [1/2, 2)
+LBMPSM_HD double from62(u64 s) {
+  const unsigned c = (unsigned)(s >> 62);
+  return of_bits((s >> (9 + c)) + ((u64)(1021u + c) << 52));
+}
+
+// ((1 + a) + b) - u and ((1 - a) + b) - u, each addition rounded: |a| < 3/8,
+// 0 <= b, u (u aligned already) below 1/12
+LBMPSM_HD void factors(double a, double b, u64 u62, double& plus, double& minus) {
+  const u64 A = align62(a), B = align62(b);
+  u64 p = rne(ONE62 + A, 10);          // in [1, 3/2): units of 2^-52
+  u64 m = rne(ONE62 - A, 9);           // in (1/2, 1]: units of 2^-53
+  p = rne53_62(rne(p + B, 10) - u62);  // still below 3/2 before the subtraction
+  m = rne53_62(rne53_62(m + B) - u62);
+  const double fp = from62(p), fm = from62(m);
+  const bool neg = (i64)bits_of(a) < 0;
+  plus = neg ? fm : fp;
+  minus = neg ? fp : fm;
+}
+
+// 1 - u, rounded (u aligned, below 1/12)
+LBMPSM_HD double one_minus(u64 u62) { return from62(rne(ONE62 - u62, 9)); }
+
+}  // namespace fx
+}  // namespace lbmpsm

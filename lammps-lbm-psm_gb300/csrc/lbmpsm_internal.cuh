@@ -435,7 +435,9 @@ struct AdjCentre {
   int weighting;
   const double* xdot;   // tangent: centre direction per image (3n); null for the adjoint
   double* out;          // adjoint: dJ/dx per image (3n)
+  double* part;         // adjoint: ADJ_CEN_PARTS partial sums of it per image
 };
+constexpr int ADJ_CEN_PARTS = 16;  // blocks per image of the centre derivative
 
 // ---------------------------------------------------------------- launchers
 // collide.cu / collide_f32.cu
