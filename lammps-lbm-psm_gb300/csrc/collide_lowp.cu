@@ -939,11 +939,10 @@ static cudaError_t multi_prepare(MultiCollide& mc, MultiMember* mem, int sm_coun
 
 cudaError_t prepare_collide_multi(MultiCollide& mc, MultiMember* mem, int storage, int sm_count) {
   if (storage == 0) {
-    // FP64: the members' own (row, x-chunk) blocks in turn
+    // FP64: the members' own blocks in turn
     int total = 0;
     for (int m = 0; m < mc.nm; ++m) {
-      const Geom& g = mem[m].p.g;
-      const long long blocks = (long long)((g.S[0] + 127) / 128) * g.S[1] * g.S[2];
+      const long long blocks = collide_f64_blocks(mem[m].p.g);
       if (total + blocks >= (1ll << 31)) return cudaErrorInvalidValue;
       mc.first[m] = total;
       total += (int)blocks;

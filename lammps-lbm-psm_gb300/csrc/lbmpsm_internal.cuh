@@ -232,7 +232,7 @@ struct CollideParams {
 // batched ensemble per box size): the blocks take tiles of one member each.
 // The row pipeline (FP32 / FP16 / BF16) packs k consecutive x-rows of a
 // storage plane into a tile, so that small boxes fill the block's threads;
-// the FP64 kernel takes the members' (row, x-chunk) blocks in turn.  Members
+// the FP64 kernel takes the members' blocks of 128 nodes in turn.  Members
 // must be 3-D and periodic on every axis.
 // FP16 storage keeps deviations scaled by 2^12; the collide kernels work on
 // the scaled values directly (a power-of-two scale commutes with rounding).
@@ -461,6 +461,7 @@ cudaError_t tune_collide_lowp(CollideParams p, int storage, int sm_count, cudaSt
 // from their geometries (host copies in members) and the device's occupancy
 cudaError_t prepare_collide_multi(MultiCollide& mc, MultiMember* members, int storage, int sm_count);
 cudaError_t launch_collide_multi(const MultiCollide& mc, int storage, int odd, cudaStream_t st);
+long long collide_f64_blocks(const Geom& g);  // 128-thread blocks of one FP64 collide
 cudaError_t launch_collide_f64_multi(const MultiCollide& mc, int odd, cudaStream_t st);
 cudaError_t launch_bc_f64(const BCParams& p, cudaStream_t st);
 cudaError_t launch_bc_f32(const BCParams& p, cudaStream_t st);
