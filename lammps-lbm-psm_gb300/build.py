@@ -37,6 +37,7 @@ def nvcc() -> str:
 def _deps(unit: str) -> list[str]:
     return [os.path.join(CSRC, unit + ".cu"), os.path.join(CSRC, "lbmpsm_internal.cuh"),
             os.path.join(CSRC, "solid_fraction.cuh"),
+            os.path.join(CSRC, "fixed_f64.cuh"),
             os.path.join(ROOT, "include", "lbmpsm.h")]
 
 

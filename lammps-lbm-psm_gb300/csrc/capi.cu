@@ -741,6 +741,9 @@ int box_setup(const lbmpsm_fix_params* p, BoxParams& bp, double& dx, double& vol
   bp.gpref_f = (float)bp.guo_pref;
   bp.tm_f = (float)(bp.tau - 0.5);
   for (int d = 0; d < 3; ++d) bp.F_f[d] = (float)bp.F[d];
+  const double x = bp.F[0], y = bp.F[1], z = bp.F[2];
+  const double eF[13] = {x, y, z, x + y, x + z, y + z, x - y, x - z, y - z, x, y, x + y, x - y};
+  for (int k = 0; k < 13; ++k) bp.eF[k] = eF[k];
   return LBMPSM_OK;
 }
 

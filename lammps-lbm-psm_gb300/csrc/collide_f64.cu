@@ -9,47 +9,36 @@
 // (src/LBM_PSM_dynamics.h:43-116), add_Fhyd (src/LBM_PSM_lattice.cpp:355-363),
 // macroCollideStream (src/LBM_PSM_BGK_dynamics.cpp:81-109), ZouHeBC
 // (src/LBM_PSM_zou_he_BC.cpp:25-398).
+#include "fixed_f64.cuh"
 #include "lbmpsm_internal.cuh"
 
 namespace lbmpsm {
 
-// signed sum of the non-zero components of e (each in {-1,0,1}) times v, in
-// axis order; equal to the reference's ex*vx + ey*vy + ez*vz for these e.
-template <int cx, int cy, int cz>
-__device__ __forceinline__ double edot(double vx, double vy, double vz) {
-  double s = 0.0;
-  bool first = true;
-  if (cx != 0) {
-    s = cx > 0 ? vx : -vx;
-    first = false;
-  }
-  if (cy != 0) {
-    if (first) {
-      s = cy > 0 ? vy : -vy;
-      first = false;
-    } else {
-      s = cy > 0 ? s + vy : s - vy;
-    }
-  }
-  if (cz != 0) {
-    if (first) {
-      s = cz > 0 ? vz : -vz;
-      first = false;
-    } else {
-      s = cz > 0 ? s + vz : s - vz;
-    }
-  }
-  return s;
+constexpr int F64_THREADS = 128, F64_BLOCKS = 5;  // (five blocks of columns fit the shared memory)
+
+// Opposite directions in pairs (q, o = opp(q)), q the one whose first non-zero
+// component is +1: e_q = +1 on axis i1, s2 on axis i2 (axis pairs: s2 = 0, i2 = i1).
+// g[a] is the index of component a of e_q in 0, +1, -1 (0, 1, 2).
+struct PairDesc {
+  int q, o, i1, i2, s2, g[3];
+};
+__constant__ PairDesc c_pairs19[9] = {
+    {1, 2, 0, 0, 0, {1, 0, 0}},   {3, 4, 1, 1, 0, {0, 1, 0}},    {5, 6, 2, 2, 0, {0, 0, 1}},
+    {7, 8, 0, 1, 1, {1, 1, 0}},   {9, 10, 0, 2, 1, {1, 0, 1}},   {11, 12, 1, 2, 1, {0, 1, 1}},
+    {13, 14, 0, 1, -1, {1, 2, 0}}, {15, 16, 0, 2, -1, {1, 0, 2}}, {17, 18, 1, 2, -1, {0, 1, 2}}};
+__constant__ PairDesc c_pairs9[4] = {{1, 3, 0, 0, 0, {1, 0, 0}},
+                                     {2, 4, 1, 1, 0, {0, 1, 0}},
+                                     {5, 7, 0, 1, 1, {1, 1, 0}},
+                                     {8, 6, 0, 1, -1, {1, 2, 0}}};
+template <class L>
+__device__ __forceinline__ const PairDesc& pair_desc(int k) {
+  return L::Q == 19 ? c_pairs19[k] : c_pairs9[k];
 }
 
-// The lattice's directions as opposite pairs (q, opp(q)), q the lower index.
-template <class L>
-struct Pairs {
-  static constexpr int N = (L::Q - 1) / 2;
-  __host__ __device__ static constexpr int q(int k) {
-    return L::Q == 19 ? 2 * k + 1 : (k < 2 ? k + 1 : k + 3);
-  }
-};
+// x with its sign turned where neg (exact)
+__device__ __forceinline__ double turned(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
 
 // a / b for three numerators: one correctly rounded reciprocal y, then per
 // quotient two corrections with exact remainders (Markstein, IBM J. Res. Dev.
@@ -57,180 +46,186 @@ struct Pairs {
 // correctly rounded quotient; the first correction makes q faithful).  Out of
 // the range where no intermediate under- or overflows (zero numerators but
 // b > 0 excepted), plain divisions.
+__device__ __forceinline__ bool is_zero(double a) {
+  return ((__double2hiint(a) & 0x7fffffff) | __double2loint(a)) == 0;
+}
 __device__ __forceinline__ bool div_range(double a) {
   const int e = (__double2hiint(a) >> 20) & 0x7ff;
-  return (e > 523 && e < 1523) || a == 0.0;
+  return (e > 523 && e < 1523) || is_zero(a);
 }
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   double q = __dmul_rn(a, y);
   q = __fma_rn(__fma_rn(-b, q, a), y, q);
   const double t = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return a == 0.0 ? a : t;
+  return is_zero(a) ? a : t;
 }
-__device__ __forceinline__ void div3(double a0, double a1, double a2, double b, double& q0,
-                                     double& q1, double& q2) {
+__device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+__device__ __forceinline__ void div3(const double (&a)[3], double b, double (&q)[3]) {
   const int e = __double2hiint(b) >> 20;  // sign and exponent: b within 2^+-100 and positive
-  if (e > 923 && e < 1123 && div_range(a0) && div_range(a1) && div_range(a2)) {
+  if (e > 923 && e < 1123 && div_range(a[0]) && div_range(a[1]) && div_range(a[2])) {
     const double y = __drcp_rn(b);
-    q0 = div_by(a0, b, y);
-    q1 = div_by(a1, b, y);
-    q2 = div_by(a2, b, y);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) q[c] = div_by(a[c], b, y);
   } else {
-    q0 = a0 / b;
-    q1 = a1 / b;
-    q2 = a2 / b;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) q[c] = div_plain(a[c], b);
   }
 }
 
-// One slot of a PSM node.
-struct Slot {
-  double B, us[3], half;  // half = 0.5*|us|^2*invCs2
-  double F[3];            // add_Fhyd: F += -B*Omega_s*e
+// The values of a block's nodes that the loop over direction pairs indexes:
+// one column per thread, so no barrier and no bank conflict.  Kept in shared
+// memory so that the loop stays rolled: unrolled over 19 directions with two
+// slots the step is 60 KB of instructions, and its warps waited for
+// instruction fetches half of the time.
+template <class L, bool FORCE>
+struct NodeCols {
+  double f[L::Q][F64_THREADS];       // populations, replaced pair by pair
+  double u[L::DIM][F64_THREADS];     // fluid velocity
+  double us[2][L::DIM][F64_THREADS]; // slot velocities
+  double F[2][L::DIM][F64_THREADS];  // slot forces
+  double t[L::Q == 9 ? 2 : 1][L::Q == 9 ? 9 : 1][F64_THREADS];  // B*Omega_s of every direction (D2Q9)
+  double g[FORCE ? 9 : 1][F64_THREADS];  // (c - u_a)*F_a at 3a + (0: c = 0, 1: c = 1, 2: c = -1)
 };
 
-// What the directions of one node share.  gF[a][c] = (c - u_a)*F_a for c = 0, 1
-// and, at index 2, -1: the products of the Guo term.
+// What the directions of one node share besides.
 struct NodeF64 {
-  double u[3], usq_half, rw[3];  // rw: rho*w of the rest, axis and diagonal weights
-  double gF[3][3], F[3];
-  double oneMinusBtot;
+  double half[3];     // 0.5*|v|^2*invCs2 of the fluid and of the slots
+  fx::u64 half62[3];  // the same aligned (fixed-point factors)
+  double rw[3];       // rho*w of the rest, axis and diagonal weights
+  double B[2], oneMinusBtot;
 };
 
-template <class L>
-__device__ __forceinline__ constexpr int weight_class(int q) {
-  return q == 0 ? 0 : (L::ex(q) * L::ex(q) + L::ey(q) * L::ey(q) + L::ez(q) * L::ez(q) == 1 ? 1 : 2);
+// e.v of a pair's first direction, from a velocity's columns
+__device__ __forceinline__ double pair_dot(const PairDesc& d, const double (*v)[F64_THREADS], int t) {
+  const double x = v[d.i1][t];
+  return d.s2 == 0 ? x : x + turned(v[d.i2][t], d.s2 < 0);
 }
 
-// Guo forcing of direction q (src/LBM_PSM_dynamics.h:102-116), scaled by
-// (1 - omega/2); g4 = (e.u)*invCs4
-template <class L, int q>
-__device__ __forceinline__ double guo_q(const NodeF64& nd, double g4, double invCs2, double pref) {
-  constexpr int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-  const double a = nd.gF[0][cx < 0 ? 2 : cx] + nd.gF[1][cy < 0 ? 2 : cy] + nd.gF[2][cz < 0 ? 2 : cz];
-  const double w = L::w(q);
-  if (q == 0) return pref * (w * (a * invCs2 + 0.0));
-  const double eF = edot<cx, cy, cz>(nd.F[0], nd.F[1], nd.F[2]);
-  return pref * (w * (a * invCs2 + (g4 * eF)));
+// The equilibria rw*(1 +- 3 e.v + 4.5 (e.v)^2 - 1.5 v.v) of a pair: e.v, its
+// multiple and its square are formed once, the opposite direction taking them
+// with the sign turned (negation is exact, so both round as when formed
+// alone; 0.5*invCs4 is exact).  FX: the sums on the integer units
+// (fixed_f64.cuh), the same bits.
+template <bool FX>
+__device__ __forceinline__ void pair_feq(double ev, double invCs2, double h4, double half,
+                                         fx::u64 half62, double rw, double& plus, double& minus) {
+  const double a = ev * invCs2, b = ev * ev * h4;
+  if (FX) {
+    fx::factors(a, b, half62, plus, minus);
+  } else {
+    plus = (1.0 + a) + b - half;
+    minus = (1.0 - a) + b - half;
+  }
+  plus = rw * plus;
+  minus = rw * minus;
 }
 
-// f after collision of direction q and its node force contributions
-// (collisionAndStream, src/LBM_PSM_BGK_dynamics.h:40-114), from feq and the
-// slots' solid equilibria f0s; NS slots (0: plain BGK).
-template <class L, int q, bool FORCE, int NS>
-__device__ __forceinline__ void relax_q(double& fq, double feq, double f0s0, double f0s1, double Fq,
-                                        const NodeF64& nd, double omega, double omo,
-                                        Slot (&sl)[2], double (&t)[2]) {
-  const double fi = fq;
+// fi after collision (collisionAndStream, src/LBM_PSM_BGK_dynamics.h:40-114)
+// with NS slots (0: plain BGK); t: B*Omega_s per slot.
+template <int NS>
+__device__ __forceinline__ double relaxed(double fi, double feq, const double (&f0s)[2],
+                                          const NodeF64& nd, double omega, double omo,
+                                          double (&t)[2]) {
   const double d = feq - fi;
-  if (NS == 0) {
-    fq = FORCE ? fi + d * omega + Fq : fi + d * omega;
-    return;
-  }
-  // one_minus_omega*(fi - feq) is -(omo*d) bit for bit
-  const double od = omo * d;
+  if (NS == 0) return fi + d * omega;
+  const double od = omo * d;  // one_minus_omega*(fi - feq) is -od bit for bit
   double r = fi + nd.oneMinusBtot * d * omega;
-  t[0] = sl[0].B * ((f0s0 - fi) - od);
-  r = r + t[0];
-  if (NS == 2) {
-    t[1] = sl[1].B * ((f0s1 - fi) - od);
-    r = r + t[1];
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    t[n] = nd.B[n] * ((f0s[n] - fi) - od);
+    r = r + t[n];
   }
-  fq = FORCE ? r + Fq : r;
+  return r;
 }
 
-template <class L, int q>
-__device__ __forceinline__ void add_force(double (&F)[3], double t) {  // F += -t*e_q
-  constexpr int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-  if (cx) F[0] = cx > 0 ? F[0] - t : F[0] + t;
-  if (cy) F[1] = cy > 0 ? F[1] - t : F[1] + t;
-  if (cz) F[2] = cz > 0 ? F[2] - t : F[2] + t;
-}
-
-// The pair k = (q, opp q): e.u, its multiple and its square are formed once,
-// the opposite direction taking them with the sign turned (negation is exact,
-// so both directions round as when formed alone); 0.5*invCs4 is exact.
-template <class L, int k, bool FORCE, int NS>
-struct CollidePairs {
-  __device__ __forceinline__ static void run(double (&f)[L::Q], const NodeF64& nd, double invCs2,
-                                             double invCs4, double omega, double omo, double pref,
-                                             Slot (&sl)[2], double (&t)[L::Q][2]) {
-    constexpr int q = Pairs<L>::q(k), o = L::opp(q);
-    constexpr int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-    const double rw = nd.rw[weight_class<L>(q)];
-    const double eu = edot<cx, cy, cz>(nd.u[0], nd.u[1], nd.u[2]);
-    const double a = eu * invCs2, b = eu * eu * (0.5 * invCs4);
-    const double ep = rw * ((1.0 + a) + b - nd.usq_half), em = rw * ((1.0 - a) + b - nd.usq_half);
-    double sp[2] = {0.0, 0.0}, sm[2] = {0.0, 0.0};
+// All directions of a node.  Guo forcing (src/LBM_PSM_dynamics.h:102-116):
+// pref*(w*(((e - u).F)*invCs2 + (e.u)*invCs4*(e.F))).
+template <class L, bool FORCE, int NS, bool FX>
+__device__ __forceinline__ void collide_dirs(NodeCols<L, FORCE>& s, int t, const NodeF64& nd,
+                                             const CollideParams& p, const BoxParams& bp,
+                                             bool has_force) {
+  const double pref = bp.guo_pref, omega = bp.omega, omo = bp.one_minus_omega;
+  const double invCs2 = p.invCs2, invCs4 = p.invCs4, h4 = 0.5 * p.invCs4;
+  auto guo = [&](int g0, int g1, int g2, double w, double last) {
+    const double a = s.g[g0][t] + s.g[3 + g1][t] + s.g[6 + g2][t];
+    return pref * (w * (a * invCs2 + last));
+  };
+  {  // the rest population
+    double f0s[2] = {0.0, 0.0}, bo[2];
+    const double feq = nd.rw[0] * (FX ? fx::one_minus(nd.half62[0]) : 1.0 - nd.half[0]);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) {  // feq(iq, rho, uSolid) (src/LBM_PSM_dynamics.h:72-85)
-      const double es = edot<cx, cy, cz>(sl[n].us[0], sl[n].us[1], sl[n].us[2]);
-      const double as = es * invCs2, bs = es * es * (0.5 * invCs4);
-      sp[n] = rw * ((1.0 + as) + bs - sl[n].half);
-      sm[n] = rw * ((1.0 - as) + bs - sl[n].half);
+    for (int n = 0; n < NS; ++n)
+      f0s[n] = nd.rw[0] * (FX ? fx::one_minus(nd.half62[1 + n]) : 1.0 - nd.half[1 + n]);
+    double r = relaxed<NS>(s.f[0][t], feq, f0s, nd, omega, omo, bo);
+    if (FORCE) r = r + guo(0, 0, 0, L::w(0), 0.0);
+    s.f[0][t] = r;
+  }
+#pragma unroll 1
+  for (int k = 0; k < (L::Q - 1) / 2; ++k) {
+    const PairDesc& d = pair_desc<L>(k);
+    const double rw = d.s2 == 0 ? nd.rw[1] : nd.rw[2];
+    const double eu = pair_dot(d, s.u, t);
+    double ep, em, sp[2] = {0.0, 0.0}, sm[2] = {0.0, 0.0}, tp[2], tm[2];
+    pair_feq<FX>(eu, invCs2, h4, nd.half[0], nd.half62[0], rw, ep, em);
+#pragma unroll
+    for (int n = 0; n < NS; ++n)  // feq(iq, rho, uSolid) (src/LBM_PSM_dynamics.h:72-85)
+      pair_feq<FX>(pair_dot(d, s.us[n], t), invCs2, h4, nd.half[1 + n], nd.half62[1 + n], rw, sp[n],
+                   sm[n]);
+    double fp = relaxed<NS>(s.f[d.q][t], ep, sp, nd, omega, omo, tp);
+    double fm = relaxed<NS>(s.f[d.o][t], em, sm, nd, omega, omo, tm);
+    if (FORCE) {
+      const double w = d.s2 == 0 ? L::w(1) : L::w(L::Q - 1);
+      const double eF = has_force ? bp.eF[(L::Q == 9 ? 9 : 0) + k] : 0.0;
+      const double last = (eu * invCs4) * eF;  // both signs turn: the same for the opposite
+      fp = fp + guo(d.g[0], d.g[1], d.g[2], w, last);
+      fm = fm + guo(d.g[0] ? 3 - d.g[0] : 0, d.g[1] ? 3 - d.g[1] : 0, d.g[2] ? 3 - d.g[2] : 0, w, last);
     }
-    const double g4 = FORCE ? eu * invCs4 : 0.0;
-    const double Fp = FORCE ? guo_q<L, q>(nd, g4, invCs2, pref) : 0.0;
-    const double Fm = FORCE ? guo_q<L, o>(nd, -g4, invCs2, pref) : 0.0;
-    relax_q<L, q, FORCE, NS>(f[q], ep, sp[0], sp[1], Fp, nd, omega, omo, sl, t[q]);
-    relax_q<L, o, FORCE, NS>(f[o], em, sm[0], sm[1], Fm, nd, omega, omo, sl, t[o]);
-    if (L::Q == 19) {  // the pairs are in direction order: add as the reference does
+    s.f[d.q][t] = fp;
+    s.f[d.o][t] = fm;
+    // node force on the particles (add_Fhyd): F += -B*Omega_s*e, in direction order
 #pragma unroll
-      for (int n = 0; n < NS; ++n) {
-        add_force<L, q>(sl[n].F, t[q][n]);
-        add_force<L, o>(sl[n].F, t[o][n]);
+    for (int n = 0; n < NS; ++n) {
+      if (L::Q == 19) {  // (the pairs are in that order)
+        s.F[n][d.i1][t] = (s.F[n][d.i1][t] - tp[n]) + tm[n];
+        if (d.s2 != 0)
+          s.F[n][d.i2][t] = (s.F[n][d.i2][t] - turned(tp[n], d.s2 < 0)) + turned(tm[n], d.s2 < 0);
+      } else {
+        s.t[n][d.q][t] = tp[n];
+        s.t[n][d.o][t] = tm[n];
       }
     }
-    CollidePairs<L, k + 1, FORCE, NS>::run(f, nd, invCs2, invCs4, omega, omo, pref, sl, t);
   }
-};
-template <class L, bool FORCE, int NS>
-struct CollidePairs<L, Pairs<L>::N, FORCE, NS> {
-  __device__ __forceinline__ static void run(double (&)[L::Q], const NodeF64&, double, double, double,
-                                             double, double, Slot (&)[2], double (&)[L::Q][2]) {}
-};
-template <class L, int q>
-struct ForceUnroll {  // in direction order, as the reference adds them
-  __device__ __forceinline__ static void run(double (&F)[3], const double (&t)[L::Q][2], int n) {
-    add_force<L, q>(F, t[q][n]);
-    ForceUnroll<L, q + 1>::run(F, t, n);
-  }
-};
-template <class L>
-struct ForceUnroll<L, L::Q> {
-  __device__ __forceinline__ static void run(double (&)[3], const double (&)[L::Q][2], int) {}
-};
-
-template <class L, bool FORCE, int NS>
-__device__ __forceinline__ void collide_dirs(double (&f)[L::Q], const NodeF64& nd,
-                                             const CollideParams& p, const BoxParams& bp,
-                                             Slot (&sl)[2]) {
-  double t[L::Q][2];
-  const double pref = bp.guo_pref, omega = bp.omega, omo = bp.one_minus_omega;
-  const double f0 = nd.rw[0] * (1.0 - nd.usq_half);
-  double s0[2] = {0.0, 0.0};
+  if (L::Q == 9) {
 #pragma unroll
-  for (int n = 0; n < NS; ++n) s0[n] = nd.rw[0] * (1.0 - sl[n].half);
-  const double F0 = FORCE ? guo_q<L, 0>(nd, 0.0, p.invCs2, pref) : 0.0;
-  relax_q<L, 0, FORCE, NS>(f[0], f0, s0[0], s0[1], F0, nd, omega, omo, sl, t[0]);
-  CollidePairs<L, 0, FORCE, NS>::run(f, nd, p.invCs2, p.invCs4, omega, omo, pref, sl, t);
-  if (L::Q != 19) {
+    for (int n = 0; n < NS; ++n) {
+      double F[2] = {0.0, 0.0};
 #pragma unroll
-    for (int n = 0; n < NS; ++n) ForceUnroll<L, 1>::run(sl[n].F, t, n);
+      for (int q = 1; q < L::Q; ++q) {
+        const double b = s.t[n][q][t];
+        if (L::ex(q)) F[0] = L::ex(q) > 0 ? F[0] - b : F[0] + b;
+        if (L::ey(q)) F[1] = L::ey(q) > 0 ? F[1] - b : F[1] + b;
+      }
+      s.F[n][0][t] = F[0];
+      s.F[n][1][t] = F[1];
+    }
   }
 }
 
 // One node of the FP64 collide + A-A stream step.
 //
 // Bound by the FP64 pipe (1.68 operations per clock and multiprocessor, the
-// memory system at a few per cent): so what directions share is formed once
-// (CollidePairs), three quotients share one reciprocal (div3), the body force
-// is a template argument, and a warp takes the plain loop when none of its
-// nodes is a PSM node, the one-slot loop when none holds two particles -- an
-// unused slot has B = 0 and adds zeros, and a node without any has 1 - B = 1,
-// so the longer loops leave its populations bit for bit as the shorter ones.
+// memory system at a few per cent), so: sums near rest run on the integer
+// units beside it (fixed_f64.cuh), what directions share is formed once
+// (pair_feq), three quotients share one reciprocal (div3), the body force is
+// a template argument, and a warp takes the plain loop when none of its nodes
+// is a PSM node, the one-slot loop when none holds two particles -- an unused
+// slot has B = 0 and adds zeros, and a node without any has 1 - B = 1, so the
+// longer loops leave its populations bit for bit as the shorter ones.
 template <class L, bool ODD, bool FORCE>
-__device__ __forceinline__ void collide_f64_node(const CollideParams& p, int sx, int sy, int sz) {
+__device__ __forceinline__ void collide_f64_node(NodeCols<L, FORCE>& s, const CollideParams& p,
+                                                 int sx, int sy, int sz) {
   constexpr int Q = L::Q;
+  const int t = threadIdx.x;
   const Geom& g = p.g;
   const long long n = node_index(g, sx, sy, sz);
   const Nbr nb = make_nbr(g, sx, sy, sz);
@@ -239,122 +234,142 @@ __device__ __forceinline__ void collide_f64_node(const CollideParams& p, int sx,
   // in place unless a separate source is given (recomputation of stored states)
   const double* Fin = p.fsrc ? static_cast<const double*>(p.fsrc) : F;
   const long long Np = g.Np;
+  const unsigned act = __activemask();
 
   const uint8_t flag = p.tab.flag[n];
-  double f[Q];
+  double rho, j[3];
+  bool near;
+  {
+    double f[Q];
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-    // incoming population q comes from the node at -e_q
-    const bool ok = nbr_ok(nb, -cx, -cy, -cz);
-    if (!ODD) {
-      f[q] = ok ? Fin[q * Np + n] : L::w(q);
-    } else {
-      const int o = nbr_off(nb, -cx, -cy, -cz);
-      f[q] = ok ? Fin[L::opp(q) * Np + n + o] : L::w(q);
+    for (int q = 0; q < Q; ++q) {
+      const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
+      // incoming population q comes from the node at -e_q
+      const bool ok = nbr_ok(nb, -cx, -cy, -cz);
+      if (!ODD) {
+        f[q] = ok ? Fin[q * Np + n] : L::w(q);
+      } else {
+        const int o = nbr_off(nb, -cx, -cy, -cz);
+        f[q] = ok ? Fin[L::opp(q) * Np + n + o] : L::w(q);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) s.f[q][t] = f[q];
+    // macro values (src/LBM_PSM_BGK_dynamics.cpp:48-77): on the integer units
+    // where every node of the warp is near rest, else in FP64
+    near = fx::macro_sums<L>(f, rho, j);
+    if (!__all_sync(act, near)) {
+      near = false;
+      rho = f[0];
+#pragma unroll
+      for (int q = 1; q < Q; ++q) rho = rho + f[q];
+      // (each sum's first term is a +e direction, taken as it is instead of 0 + f)
+      j[0] = f[1];
+      j[1] = f[Q == 19 ? 3 : 2];
+      j[2] = Q == 19 ? f[5] : 0.0;
+#pragma unroll
+      for (int q = 2; q < Q; ++q) {
+        const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
+        if (cx) j[0] = cx > 0 ? j[0] + f[q] : j[0] - f[q];
+        if (cy && q > (Q == 19 ? 3 : 2)) j[1] = cy > 0 ? j[1] + f[q] : j[1] - f[q];
+        if (cz && q > 5) j[2] = cz > 0 ? j[2] + f[q] : j[2] - f[q];
+      }
     }
   }
-
-  // macro values (src/LBM_PSM_BGK_dynamics.cpp:48-77)
-  double rho = f[0];
 #pragma unroll
-  for (int q = 1; q < Q; ++q) rho = rho + f[q];
-  // (each sum's first term is a +e direction, taken as it is instead of 0 + f)
-  double j[3] = {f[1], f[L::Q == 19 ? 3 : 2], L::Q == 19 ? f[5] : 0.0};
-#pragma unroll
-  for (int q = 2; q < Q; ++q) {
-    const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-    if (cx) j[0] = cx > 0 ? j[0] + f[q] : j[0] - f[q];
-    if (cy && q > (L::Q == 19 ? 3 : 2)) j[1] = cy > 0 ? j[1] + f[q] : j[1] - f[q];
-    if (cz && q > 5) j[2] = cz > 0 ? j[2] + f[q] : j[2] - f[q];
-  }
-  NodeF64 nd;
-  if (FORCE) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      j[c] = j[c] + bp.F[c] * 0.5;
-      nd.F[c] = bp.has_force ? bp.F[c] : 0.0;  // (a box of an ensemble may have none)
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)  // (|F|^2 of a non-zero F may underflow to "no force")
-      if ((__double_as_longlong(bp.F[c]) << 1) != 0ll) j[c] = j[c] + bp.F[c] * 0.5;
-  }
-  div3(j[0], j[1], j[2], rho, nd.u[0], nd.u[1], nd.u[2]);
+  for (int c = 0; c < 3; ++c)  // (|F|^2 of a non-zero F may underflow to "no force")
+    if (FORCE || !is_zero(bp.F[c])) j[c] = j[c] + bp.F[c] * 0.5;
+  double u[3];
+  div3(j, rho, u);
   if (p.store_macro) {
     p.rho_out[n] = rho;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) p.u_out[3 * n + c] = nd.u[c];
+    for (int c = 0; c < 3; ++c) p.u_out[3 * n + c] = u[c];
   }
-  nd.usq_half = 0.5 * (nd.u[0] * nd.u[0] + nd.u[1] * nd.u[1] + nd.u[2] * nd.u[2]) * p.invCs2;
+  NodeF64 nd;
+  nd.half[0] = 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]) * p.invCs2;
+  nd.half62[0] = fx::align62(nd.half[0]);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) nd.rw[c] = rho * L::w(c == 0 ? 0 : (c == 1 ? 1 : Q - 1));
+  for (int c = 0; c < 3; ++c) {
+    near = near && fx::slow(u[c]);
+    if (c < L::DIM) s.u[c][t] = u[c];
+    nd.rw[c] = rho * L::w(c == 0 ? 0 : (c == 1 ? 1 : Q - 1));
+  }
+  const bool has_force = FORCE && bp.has_force != 0;  // (a box of an ensemble may have none)
   if (FORCE) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      nd.gF[c][0] = (0.0 - nd.u[c]) * nd.F[c];
-      nd.gF[c][1] = (1.0 - nd.u[c]) * nd.F[c];
-      nd.gF[c][2] = (-1.0 - nd.u[c]) * nd.F[c];
+      const double Fc = has_force ? bp.F[c] : 0.0;
+      s.g[3 * c][t] = (0.0 - u[c]) * Fc;
+      s.g[3 * c + 1][t] = (1.0 - u[c]) * Fc;
+      s.g[3 * c + 2][t] = (-1.0 - u[c]) * Fc;
     }
   }
-  nd.oneMinusBtot = 1.0;
 
-  const unsigned act = __activemask();
   const bool psm = flag != 0;
-  Slot sl[2];
   if (!__any_sync(act, psm)) {
-    collide_dirs<L, FORCE, 0>(f, nd, p, bp, sl);
+    if (__all_sync(act, near))
+      collide_dirs<L, FORCE, 0, true>(s, t, nd, p, bp, has_force);
+    else
+      collide_dirs<L, FORCE, 0, false>(s, t, nd, p, bp, has_force);
   } else {
+    int2 id = make_int2(0, 0);
+    double2 e = make_double2(0.0, 0.0);
+    if (psm) {
+      id = p.tab.ids[n];
+      e = p.tab.eps[n];
+    }
+    const bool has[2] = {id.x > 0, id.y > 0};
+    double B1 = has[0] ? e.x : 0.0;
+    double B2 = has[1] ? e.y : 0.0;
+    if (p.weighting == 1) {  // Noble-Torczynski weighting (opt-in)
+      const double tm = bp.tau - 0.5;
+      if (has[0]) B1 = B1 * tm / ((1.0 - B1) + tm);
+      if (has[1]) B2 = B2 * tm / ((1.0 - B2) + tm);
+    }
+    double Btot = B1 + B2;
+    if (Btot > 1.0) {
+      B1 = B1 / Btot;
+      B2 = B2 / Btot;
+      Btot = 1.0;
+    }
+    nd.B[0] = B1;
+    nd.B[1] = B2;
+    nd.oneMinusBtot = 1.0 - Btot;
+    const double* us = p.tab.us + 6 * n;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      sl[k].B = 0.0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) sl[k].us[c] = sl[k].F[c] = 0.0;
-      sl[k].half = 0.0;
-    }
-    if (psm) {
-      const int2 id = p.tab.ids[n];
-      const double2 e = p.tab.eps[n];
-      const double* us = p.tab.us + 6 * n;
-      const bool has1 = id.x > 0, has2 = id.y > 0;
-      double B1 = has1 ? e.x : 0.0;
-      double B2 = has2 ? e.y : 0.0;
-      if (p.weighting == 1) {  // Noble-Torczynski weighting (opt-in)
-        const double tm = bp.tau - 0.5;
-        if (has1) B1 = B1 * tm / ((1.0 - B1) + tm);
-        if (has2) B2 = B2 * tm / ((1.0 - B2) + tm);
-      }
-      double Btot = B1 + B2;
-      if (Btot > 1.0) {
-        B1 = B1 / Btot;
-        B2 = B2 / Btot;
-        Btot = 1.0;
-      }
-      sl[0].B = B1;
-      sl[1].B = B2;
-      nd.oneMinusBtot = 1.0 - Btot;
+      double v[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        if (has1) sl[0].us[c] = us[c];
-        if (has2) sl[1].us[c] = us[3 + c];
+        v[c] = has[k] ? us[3 * k + c] : 0.0;
+        if (c < L::DIM) {
+          s.us[k][c][t] = v[c];
+          s.F[k][c][t] = 0.0;
+        }
+        near = near && fx::slow(v[c]);
       }
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-        sl[k].half = 0.5 *
-                     (sl[k].us[0] * sl[k].us[0] + sl[k].us[1] * sl[k].us[1] + sl[k].us[2] * sl[k].us[2]) *
-                     p.invCs2;
+      nd.half[1 + k] = 0.5 * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * p.invCs2;
+      nd.half62[1 + k] = fx::align62(nd.half[1 + k]);
     }
-    if (!__any_sync(act, (flag & 2) != 0))
-      collide_dirs<L, FORCE, 1>(f, nd, p, bp, sl);
-    else
-      collide_dirs<L, FORCE, 2>(f, nd, p, bp, sl);
+    const bool one = !__any_sync(act, (flag & 2) != 0);
+    if (__all_sync(act, near)) {
+      if (one)
+        collide_dirs<L, FORCE, 1, true>(s, t, nd, p, bp, has_force);
+      else
+        collide_dirs<L, FORCE, 2, true>(s, t, nd, p, bp, has_force);
+    } else {
+      if (one)
+        collide_dirs<L, FORCE, 1, false>(s, t, nd, p, bp, has_force);
+      else
+        collide_dirs<L, FORCE, 2, false>(s, t, nd, p, bp, has_force);
+    }
     if (psm) {
       double* nf = static_cast<double*>(p.tab.nodeF) + 6 * n;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        nf[c] = sl[0].F[c];
-        nf[3 + c] = sl[1].F[c];
-      }
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) nf[3 * k + c] = c < L::DIM ? s.F[k][c < L::DIM ? c : 0][t] : 0.0;
     }
   }
 
@@ -362,9 +377,9 @@ __device__ __forceinline__ void collide_f64_node(const CollideParams& p, int sx,
   for (int q = 0; q < Q; ++q) {
     const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
     if (!ODD) {
-      F[L::opp(q) * Np + n] = f[q];
+      F[L::opp(q) * Np + n] = s.f[q][t];
     } else {
-      if (nbr_ok(nb, cx, cy, cz)) F[q * Np + n + nbr_off(nb, cx, cy, cz)] = f[q];
+      if (nbr_ok(nb, cx, cy, cz)) F[q * Np + n + nbr_off(nb, cx, cy, cz)] = s.f[q][t];
     }
   }
 }
@@ -372,7 +387,6 @@ __device__ __forceinline__ void collide_f64_node(const CollideParams& p, int sx,
 // Node of thread t of block b when the stored nodes (x fastest, without the
 // rows' padding) are dealt out 128 to a block: rows shorter than a block, or
 // not a multiple of a warp, leave no lane of the FP64 pipe idle.
-constexpr int F64_THREADS = 128;
 __device__ __forceinline__ bool node_of(const Geom& g, unsigned b, int& sx, int& sy, int& sz) {
   const unsigned S0 = (unsigned)g.S[0];
   const unsigned first = b * (unsigned)F64_THREADS;  // the node count stays below 2^32 (memory)
@@ -389,24 +403,26 @@ __device__ __forceinline__ bool node_of(const Geom& g, unsigned b, int& sx, int&
 }
 
 template <class L, bool ODD, bool FORCE>
-__global__ void __launch_bounds__(F64_THREADS) collide_f64_kernel(CollideParams p) {
+__global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_kernel(CollideParams p) {
+  __shared__ NodeCols<L, FORCE> s;
   int sx, sy, sz;
   if (!node_of(p.g, blockIdx.x, sx, sy, sz)) return;
-  collide_f64_node<L, ODD, FORCE>(p, sx, sy, sz);
+  collide_f64_node<L, ODD, FORCE>(s, p, sx, sy, sz);
 }
 
 // The members of a group in one launch: member m owns blocks
 // [first[m], first[m+1]), laid out as its own kernel's; every node runs the
 // same code as above, so the results are the members'.
 template <class L, bool ODD, bool FORCE>
-__global__ void __launch_bounds__(F64_THREADS) collide_f64_multi_kernel(MultiCollide mc) {
+__global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_multi_kernel(MultiCollide mc) {
+  __shared__ NodeCols<L, FORCE> s;
   const int b = blockIdx.x;
   int m = 0;
   while (m + 1 < mc.nm && b >= mc.first[m + 1]) ++m;
   const CollideParams& p = mc.m[m].p;
   int sx, sy, sz;
   if (!node_of(p.g, (unsigned)(b - mc.first[m]), sx, sy, sz)) return;
-  collide_f64_node<L, ODD, FORCE>(p, sx, sy, sz);
+  collide_f64_node<L, ODD, FORCE>(s, p, sx, sy, sz);
 }
 
 long long collide_f64_blocks(const Geom& g) {

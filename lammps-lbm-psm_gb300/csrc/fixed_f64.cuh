@@ -4,14 +4,14 @@
 // This GPU issues 1.68 FP64 operations per clock and multiprocessor against
 // about 100 integer ones, and both at once, so an addition whose rounding
 // position is known can be had for a dozen integer instructions beside the
-// FP64 pipe.  Near equilibrium it is known: populations, their sums and the
-// factors 1 + 3 e.u + ... of the equilibria keep to one or two binades.  The
-// values are held as 64-bit integers in units of 2^-60 (populations and
-// sums) or 2^-62 (the factors); each result is rounded to 53 significant bits,
-// ties to even, as the IEEE addition it stands for.  Every function states
-// the range it needs; the caller checks the ranges (populations in
-// [2^-6, 1), velocity components below 1/16 and the sums below) and takes the
-// FP64 expressions otherwise.
+// FP64 pipe.  Near rest it is known: populations, their sums and the factors
+// 1 + 3 e.u + ... of the equilibria keep to a few binades.  The values are held
+// as 64-bit integers in units of 2^-61 (populations and sums) or 2^-62 (the
+// factors); each result is rounded to 53 significant bits, ties to even, as
+// the IEEE addition it stands for.  Every function states the range it needs;
+// the caller checks the ranges (populations in [2^-7, 1), densities above 0.9
+// and below 2, velocity components below 5/64) and takes the FP64 expressions
+// otherwise.  A suspension whose spheres move at 0.04 stays inside.
 //
 // Host compilable: the functions are compared with IEEE arithmetic on the CPU.
 #pragma once
@@ -49,6 +49,13 @@ LBMPSM_HD double of_bits(u64 b) {
   return x;
 #endif
 }
+LBMPSM_HD int clz32(unsigned x) {  // x != 0
+#ifdef __CUDA_ARCH__
+  return __clz((int)x);
+#else
+  return __builtin_clz(x);
+#endif
+}
 LBMPSM_HD int clz64(u64 x) {  // x != 0
 #ifdef __CUDA_ARCH__
   return __clzll((i64)x);
@@ -57,15 +64,15 @@ LBMPSM_HD int clz64(u64 x) {  // x != 0
 #endif
 }
 
-// f in units of 2^-60; f in [2^-6, 1), else bad becomes non-zero.  The result
+// f in units of 2^-61; f in [2^-7, 1), else bad becomes non-zero.  The result
 // is a multiple of 4.
-LBMPSM_HD u64 to60(double f, unsigned& bad) {
+LBMPSM_HD u64 to61(double f, unsigned& bad) {
   const u64 b = bits_of(f);
   const unsigned hi = (unsigned)(b >> 32);
-  const unsigned s = (hi >> 20) - (1023u - 6u);  // 0..5; sign, small, large, inf, NaN: beyond
-  bad |= s > 5u ? 1u : 0u;
+  const unsigned s = (hi >> 20) - (1023u - 7u);  // 0..6; sign, small, large, inf, NaN: beyond
+  bad |= s > 6u ? 1u : 0u;
   const u64 m = ((u64)((hi & 0xFFFFFu) | 0x100000u) << 32) | (b & 0xFFFFFFFFull);
-  return m << ((s + 2u) & 7u);
+  return m << ((s + 2u) & 15u);
 }
 
 // t rounded to a multiple of 2^sh, ties to even (t >= 0)
@@ -73,39 +80,41 @@ LBMPSM_HD u64 rne(u64 t, int sh) {
   return (t + ((1ull << (sh - 1)) - 1ull) + ((t >> sh) & 1ull)) & ~((1ull << sh) - 1ull);
 }
 
-// t >= 0 in units of 2^-60, rounded to 53 bits: t in [2^(58+k0), 2^(60+k0))
+// t >= 0 in units of 2^-61, rounded to 53 bits: t in [2^(59+k0), 2^(61+k0))
 // where k0 = 0 (t in [1/4, 1)) or 1 (t in [1/2, 2))
 LBMPSM_HD u64 rne53_of2(u64 t, int k0) {
-  const unsigned c = (unsigned)(t >> (59 + k0)) & 1u;
-  const int sh = 6 + k0 + (int)c;
-  const u64 half = 32ull << (k0 + (int)c);
+  const unsigned c = (unsigned)(t >> (60 + k0)) & 1u;
+  const int sh = 7 + k0 + (int)c;
+  const u64 half = 64ull << (k0 + (int)c);
   return (t + (half - 1ull) + ((t >> sh) & 1ull)) & ~(2ull * half - 1ull);
 }
 
-// t (a multiple of 4, |t| < 2^57, units of 2^-60) rounded to 53 bits
+// high word of |t| (of |t| - 1 for negative t)
+LBMPSM_HD unsigned abs_hi(i64 t) { return (unsigned)((u64)t >> 32) ^ (unsigned)(t >> 63); }
+
+// t (a multiple of 4, |t| < 2^62) rounded to 53 bits: multiples of 4 below
+// 2^55 are held exactly (and left alone by the rounding to 2^2)
 LBMPSM_HD i64 rne53_signed(i64 t) {
-  const unsigned a = (unsigned)(((u64)t >> 32) ^ (u64)(i64)(t >> 63));  // high word of |t| (or |t| - 1)
-  const unsigned m = a >= (1u << 24) ? 15u : (a >= (1u << 23) ? 7u : 0u);
-  const int sh = a >= (1u << 24) ? 4 : 3;
-  const unsigned low = (unsigned)t;
-  const u64 inc = (u64)((m >> 1) + ((low >> sh) & 1u & m));
+  const int sh = 2 + (9 - clz32(abs_hi(t) | 0x400000u));
+  const unsigned m = (1u << sh) - 1u;
+  const u64 inc = (u64)((m >> 1) + (((unsigned)t >> sh) & 1u));
   return (i64)(((u64)t + inc) & ~(u64)m);
 }
 
-// the double t * 2^-60 (t with at most 53 significant bits)
-LBMPSM_HD double from60(i64 t) {
+// the double t * 2^-61 (t with at most 53 significant bits)
+LBMPSM_HD double from61(i64 t) {
   const u64 sg = (u64)t & 0x8000000000000000ull;
   const u64 a = t < 0 ? (u64)0 - (u64)t : (u64)t;
   if (a == 0) return 0.0;
   const int lz = clz64(a);
   const u64 m = (a << lz) >> 11;  // 53 bits, the leading one at bit 52
-  return of_bits(sg | (m + ((u64)(1025 - lz) << 52)));
+  return of_bits(sg | (m + ((u64)(1024 - lz) << 52)));
 }
 
-// the double t * 2^-60 for a 53-bit t in [1/2, 2)
-LBMPSM_HD double from60_near1(u64 t) {
-  const unsigned c = (unsigned)(t >> 60);
-  return of_bits((t >> (7 + c)) + ((u64)(1021u + c) << 52));
+// the double t * 2^-61 for a 53-bit t in [1/2, 2)
+LBMPSM_HD double from61_near1(u64 t) {
+  const unsigned c = (unsigned)(t >> 61);
+  return of_bits((t >> (8 + c)) + ((u64)(1021u + c) << 52));
 }
 
 // |x| in units of 2^-62, |x| < 1/2: bits below the unit are kept as a set
@@ -136,13 +145,14 @@ LBMPSM_HD double from62(u64 s) {
   return of_bits((s >> (9 + c)) + ((u64)(1021u + c) << 52));
 }
 
-// ((1 + a) + b) - u and ((1 - a) + b) - u, each addition rounded: |a| < 3/8,
-// 0 <= b, u (u aligned already) below 1/12
+// ((1 + a) + b) - u and ((1 - a) + b) - u, each addition rounded, for a = 3 x,
+// b = 4.5 x^2 with |x| <= 5/32 and 0 <= u < 1/24 (u aligned already): the first
+// stays in [1 - u, 3/2 + u], the second in [3/5 - u, 1]
 LBMPSM_HD void factors(double a, double b, u64 u62, double& plus, double& minus) {
   const u64 A = align62(a), B = align62(b);
   u64 p = rne(ONE62 + A, 10);          // in [1, 3/2): units of 2^-52
   u64 m = rne(ONE62 - A, 9);           // in (1/2, 1]: units of 2^-53
-  p = rne53_62(rne(p + B, 10) - u62);  // still below 3/2 before the subtraction
+  p = rne53_62(rne(p + B, 10) - u62);  // (in [1, 2) before the subtraction)
   m = rne53_62(rne53_62(m + B) - u62);
   const double fp = from62(p), fm = from62(m);
   const bool neg = (i64)bits_of(a) < 0;
@@ -150,8 +160,64 @@ LBMPSM_HD void factors(double a, double b, u64 u62, double& plus, double& minus)
   minus = neg ? fp : fm;
 }
 
-// 1 - u, rounded (u aligned, below 1/12)
+// 1 - u, rounded (u aligned, below 1/24)
 LBMPSM_HD double one_minus(u64 u62) { return from62(rne(ONE62 - u62, 9)); }
+
+// Density and momentum sums of compute_macro_values
+// (src/LBM_PSM_BGK_dynamics.cpp:48-77), each addition rounded in its place:
+// rho = ((f0 + f1) + f2) + ..., j_a the signed sum over the directions with a
+// component along a.  Returns whether every range held (else the outputs are
+// not to be used): populations in [2^-7, 1), the sum of the first two (D3Q19:
+// the first two in [1/4, 1/2), the first three below 1/2; the first five) at
+// least 1/2, the density below 2, the partial sums of j below 1/4.
+template <class L>
+LBMPSM_HD bool macro_sums(const double* f, double& rho, double (&j)[3]) {
+  constexpr int Q = L::Q;
+  u64 F[Q];
+  unsigned bad = 0;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) F[q] = to61(f[q], bad);
+  u64 t = F[0];
+#pragma unroll
+  for (int q = 1; q < Q; ++q) {
+    t += F[q];
+    if (Q == 19) {
+      // at rest 7/18, 8/18 | 1/2 | 5/9 .. 1
+      if (q == 1) bad |= t < (1ull << 59) ? 1u : 0u;
+      if (q == 2) bad |= t >= (1ull << 60) ? 1u : 0u;
+      if (q == 4) bad |= t < (1ull << 60) || t >= (1ull << 61) ? 1u : 0u;
+      t = q <= 2 ? rne(t, 7) : rne53_of2(t, q == 3 ? 0 : 1);
+    } else {
+      // at rest 5/9 .. 1
+      if (q == 1) bad |= t < (1ull << 60) ? 1u : 0u;
+      t = rne53_of2(t, 1);
+    }
+  }
+  bad |= t >= (1ull << 62) ? 1u : 0u;
+  rho = from61_near1(t);
+  unsigned over = 0;  // high words of the partial sums
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    j[a] = 0.0;
+    if (a == 2 && Q == 9) continue;
+    i64 s = 0;
+    int terms = 0;
+#pragma unroll
+    for (int q = 1; q < Q; ++q) {
+      const int c = a == 0 ? L::ex(q) : (a == 1 ? L::ey(q) : L::ez(q));
+      if (c == 0) continue;
+      s = c > 0 ? s + (i64)F[q] : s - (i64)F[q];
+      if (++terms == 1) continue;  // one population: exact
+      over |= abs_hi(s);
+      s = rne53_signed(s);
+    }
+    j[a] = from61(s);
+  }
+  return (bad | (over >> 27)) == 0;
+}
+
+// |x| < 5/64 (false for inf and NaN)
+LBMPSM_HD bool slow(double x) { return ((unsigned)(bits_of(x) >> 32) & 0x7FFFFFFFu) < 0x3FB40000u; }
 
 }  // namespace fx
 }  // namespace lbmpsm

@@ -197,6 +197,9 @@ struct BoxParams {
   double origin[3];                              // the box's own frame
   double Uc, u_lb, tc, dt_d;                     // UnitConversion
   double forceFactor, torqueFactor;
+  // e.F of the FP64 collide's direction pairs: nine of D3Q19 (x, y, z, x+y,
+  // x+z, y+z, x-y, x-z, y-z), then four of D2Q9 (x, y, x+y, x-y)
+  double eF[13];
 };
 
 // launch shape of the row-pipelined FP32/FP16 collide kernel (grid 0: the
