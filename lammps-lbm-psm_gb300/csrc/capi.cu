@@ -615,6 +615,7 @@ int enqueue_post(lbmpsm_handle* h, int n, bool bc) {
     rp.S2 = h->out2[2];
     rp.status = h->d_status;
     rp.status_out = h->host_direct ? &h->status_host : nullptr;
+    rp.sm_count = h->sm_count;
     CUDA_TRY(h, launch_reduce(rp, h->stream));
   }
   if (bc_aside) CUDA_TRY(h, cudaStreamWaitEvent(h->stream, h->ev_bc_join, 0));
@@ -1173,7 +1174,7 @@ int device_step(lbmpsm_handle* h, int n, const int* tag, const double* x, const 
     if (e == cudaSuccess) e = cudaGraphGetNodes(graph, nodes.data(), &nn);
     cudaGraphNode_t gn = nullptr, rn = nullptr;
     const void* fg = img_prep_fn();
-    const void* fr = reduce_fn(h->opt.storage == LBMPSM_STORAGE_FP64 ? 1 : 0);
+    const void* fr = reduce_fn(h->opt.storage == LBMPSM_STORAGE_FP64 ? 1 : 0, n, h->sm_count);
     for (size_t k = 0; e == cudaSuccess && k < nn; ++k) {
       cudaGraphNodeType ty;
       if (cudaGraphNodeGetType(nodes[k], &ty) != cudaSuccess || ty != cudaGraphNodeTypeKernel) continue;

@@ -372,6 +372,7 @@ struct ReduceParams {
   double* S2;         // of lbmpsm_step), written with the first
   const int* status;  // the step's status word (device)
   int* status_out;    // optional host-visible copy of it, written by block 0 last
+  int sm_count;       // multiprocessors
 };
 
 // status bits
@@ -487,7 +488,7 @@ cudaError_t launch_map(const MapParams& p, cudaStream_t st, cudaStream_t aux = n
 cudaError_t launch_reduce(const ReduceParams& p, cudaStream_t st);
 // the kernels whose arguments a replayed device-step graph updates per call
 const void* img_prep_fn();
-const void* reduce_fn(int nodeF_is_double);
+const void* reduce_fn(int nodeF_is_double, int n, int sm_count);
 cudaError_t launch_table_export(const Geom& g, const Table& t, int* ids, double* eps,
                                 double* us, cudaStream_t st);
 cudaError_t launch_export_fields(const Geom& g, const Table& t, const double* rho,

@@ -20,13 +20,18 @@
 // FP64 expression, so the count is the reference's count.
 //
 // Reduce (replaces calculateHydrodynamicInteractions,
-// src/LBM_PSM_exchangeParticleData.cpp:172-244): one block per image sums
-// the node forces of its tag over the box clamped to interior nodes, with a
-// fixed-order warp-shuffle and block reduction (deterministic run to run).
+// src/LBM_PSM_exchangeParticleData.cpp:172-244): the node forces of an image's
+// tag summed over the box clamped to interior nodes in a fixed order
+// (deterministic run to run).
+#include <cooperative_groups.h>
+
 #include "lbmpsm_internal.cuh"
 #include "solid_fraction.cuh"
 
 namespace lbmpsm {
+
+// Whether n images are too few to fill the device with one block each.
+static bool few_images(int n, int sm_count) { return n < sm_count; }
 
 static __device__ __forceinline__ int clampi(int v, int lo, int hi) {
   return v < lo ? lo : (v > hi ? hi : v);
@@ -390,18 +395,24 @@ static __device__ __forceinline__ int corner_count(int dim, float dxf, float dyf
 constexpr int SFC_THREADS = 64;   // classification: one block per image
 constexpr int SFS_THREADS = 128;  // shell counting: persistent warps
 
-// Phase 1 of the map, one block per image.  The box's codes are first set
-// to 0 with coalesced stores; then only the nodes of each x-row that may
-// lie within rP (an FP32 bound widened by 0.01 node: a superset of the
-// nodes classify_node does not put beyond rP for certain) are classified by
-// the early-out radii of calcSolidFraction.  Inside nodes get their code
-// here, and so do shell nodes whose sub-cells all lie on one side of the
-// surface; the other shell nodes (whose sub-cells must be counted) are
-// queued per warp in shared memory and appended to a global list with one
-// atomic per flush.  Each warp takes 32 rows at a time, one per lane, and
-// walks the nodes of their segments 32 at a time (consecutive lanes on
-// consecutive nodes of a row).
+// Phase 1 of the map.  An image's box is walked in groups of x-rows, one warp
+// a group.  The warp first sets the group's codes to 0 with coalesced stores;
+// then only the nodes of each row that may lie within rP (an FP32 bound
+// widened by 0.01 node: a superset of the nodes classify_node does not put
+// beyond rP for certain) are classified by the early-out radii of
+// calcSolidFraction.  Inside nodes get their code here, and so do shell nodes
+// whose sub-cells all lie on one side of the surface; the other shell nodes
+// (whose sub-cells must be counted) are queued per warp in shared memory and
+// appended to a global list with one atomic per flush.  The rows' segments go
+// one per lane, and the warp walks their nodes 32 at a time (consecutive lanes
+// on consecutive nodes of a row).
+//
+// With many images one block of two warps each, 32 rows a group (2260 images
+// of diameter 12: one wave); with few, an image's groups of 8 rows are dealt
+// to SFC_PARTS blocks (one image of diameter 16 by one block: 30 us).
 constexpr int SFC_QW = 256;  // per-warp queue of shell nodes
+constexpr int SFC_PARTS = 16;
+template <int ROWS>
 __global__ void __launch_bounds__(SFC_THREADS) sf_classify_kernel(MapParams p) {
   const Img& im = p.img[blockIdx.x];
   if (!im.valid) return;
@@ -413,10 +424,7 @@ __global__ void __launch_bounds__(SFC_THREADS) sf_classify_kernel(MapParams p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Geom& g = p.g;
   const int wx = im.box[0], wy = im.box[1], wz = im.box[2];
-  const int vol = wx * wy * wz;
   unsigned short* code = p.sfcode + im.sf_off;
-  for (int li = threadIdx.x; li < vol; li += SFC_THREADS) code[li] = 0;
-  __syncthreads();  // the zeros land before any code of this block
   // reference-frame coordinates of the box's first node
   const int h0 = im.lo[0] + g.off[0], h1 = im.lo[1] + g.off[1];
   const int h2 = im.lo[2] - im.zoff + g.off[2];  // z in the box's own frame
@@ -438,10 +446,12 @@ __global__ void __launch_bounds__(SFC_THREADS) sf_classify_kernel(MapParams p) {
     qn = 0;
   };
   const int R = wy * wz;
-  for (int r0 = warp * 32; r0 < R; r0 += SFC_THREADS) {
+  for (int r0 = ((int)blockIdx.y * NW + warp) * ROWS; r0 < R; r0 += (int)gridDim.y * NW * ROWS) {
     const int r = r0 + lane;
+    for (int li = r0 * wx + lane; li < min(R, r0 + ROWS) * wx; li += 32) code[li] = 0;
+    __syncwarp();  // the zeros land before any code of the group
     int xa = 0, len = 0, by = 0, bz = 0;
-    if (r < R) {
+    if (lane < ROWS && r < R) {
       bz = (int)fast_div((unsigned)r, fy);
       by = r - bz * wy;
       const float dy = small_int_to_float(h1 + by - im.xi[1]) - im.xf[1];
@@ -834,7 +844,10 @@ cudaError_t launch_map(const MapParams& p, cudaStream_t st, cudaStream_t aux, cu
   cell_scan_kernel<<<1, SCAN_THREADS, 0, cl>>>(p.cell_count, p.cell_off, ncells);
   img_fill_kernel<<<wblocks, tb, 0, cl>>>(p);
   cell_sort_kernel<<<(ncells + 255) / 256, 256, 0, cl>>>(p, ncells);
-  sf_classify_kernel<<<p.n, SFC_THREADS, 0, st>>>(p);
+  if (few_images(p.n, p.sm_count))
+    sf_classify_kernel<8><<<dim3((unsigned)p.n, SFC_PARTS), SFC_THREADS, 0, st>>>(p);
+  else
+    sf_classify_kernel<32><<<p.n, SFC_THREADS, 0, st>>>(p);
   sf_shell_kernel<<<p.sm_count * 8, SFS_THREADS, 0, st>>>(p);
   if (two) {
     if ((e = cudaEventRecord(join, aux)) != cudaSuccess) return e;
@@ -853,110 +866,11 @@ cudaError_t launch_map(const MapParams& p, cudaStream_t st, cudaStream_t aux, cu
 }
 
 // ------------------------------------------------------------------ reduce
-constexpr int RED_THREADS = 128;
-
-// Node (i, j, k) lies beyond the early-out radius rP of the image for
-// certain (FP32 distance with the margin proven for classify_node), so its
-// solid fraction for this image is 0.
-static __device__ __forceinline__ bool beyond_rP(const Img& im, int i, int j, int k) {
-  const float u = 5.9604644775390625e-08f;  // 2^-24
-  const float dx = small_int_to_float(i - im.xi[0]) - im.xf[0];
-  const float dy = small_int_to_float(j - im.xi[1]) - im.xf[1];
-  const float dz = small_int_to_float(k - im.xi[2]) - im.xf[2];
-  const float d32 = dx * dx + dy * dy + dz * dz;
-  const float m = 16.0f * u * (5.0f * d32 + 2.0f * (fabsf(dx) + fabsf(dy) + fabsf(dz)) + 1.0f + im.rP2f);
-  return d32 > im.rP2f + m;
-}
-
 // The step's status word into host memory for the host-pointer step (every
 // kernel that sets a bit ran before the reduction in stream order).
 static __device__ __forceinline__ void copy_status(const ReduceParams& p) {
   if (p.status_out && blockIdx.x == 0 && threadIdx.x == 0)
     *p.status_out = *static_cast<const volatile int*>(p.status);
-}
-
-static __device__ __forceinline__ void block_reduce_store(double (&acc)[12], const ReduceParams& p,
-                                                          int ip) {
-  // fixed-order reduction: butterfly within warps, then warps in index order
-#pragma unroll
-  for (int k = 0; k < 12; ++k)
-    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  __shared__ double part[RED_THREADS / 32][12];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-    for (int k = 0; k < 12; ++k) part[warp][k] = acc[k];
-  __syncthreads();
-  if (threadIdx.x < 12) {
-    const int k = threadIdx.x;
-    double sum = 0.0;
-    for (int w = 0; w < RED_THREADS / 32; ++w) sum += part[w][k];
-    if (k < 3) {
-      p.fh[3 * ip + k] = sum;
-      if (p.fh2) p.fh2[3 * ip + k] = sum;
-    } else if (k < 6) {
-      p.th[3 * ip + (k - 3)] = sum;
-      if (p.th2) p.th2[3 * ip + (k - 3)] = sum;
-    } else {
-      p.S[6 * ip + (k - 6)] = -sum;
-      if (p.S2) p.S2[6 * ip + (k - 6)] = -sum;
-    }
-  }
-}
-
-// FP64 node forces (FP64 storage): the reference's per-node terms in FP64.
-__global__ void __launch_bounds__(RED_THREADS) reduce_f64_kernel(ReduceParams p) {
-  const int ip = blockIdx.x;
-  const Geom& g = p.g;
-  const int tag = p.tag[ip];
-  const Img& bx = p.img[ip];  // box and centre from the map's image record
-  const int wx = bx.qhi[0] - bx.qlo[0], wy = bx.qhi[1] - bx.qlo[1], wz = bx.qhi[2] - bx.qlo[2];
-  double acc[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) acc[k] = 0.0;
-  if (wx > 0 && wy > 0 && wz > 0) {
-    const long long total = (long long)wx * wy * wz;
-    const double ff = p.box[bx.bidx].forceFactor, tf = p.box[bx.bidx].torqueFactor;
-    const double* nodeF = static_cast<const double*>(p.tab.nodeF);
-    // x fastest: consecutive threads read consecutive nodes
-    const FastDiv fx = make_fastdiv((unsigned)wx), fy = make_fastdiv((unsigned)wy);
-    for (long long t = threadIdx.x; t < total; t += RED_THREADS) {
-      const int q1 = (int)fast_div((unsigned)t, fx);
-      const int q2 = (int)fast_div((unsigned)q1, fy);
-      const int i = bx.qlo[0] + (int)t - q1 * wx;
-      const int j = bx.qlo[1] + q1 - q2 * wy;
-      const int k = bx.qlo[2] + q2;
-      if (bx.solo && beyond_rP(bx, i, j, k)) continue;
-      const long long n = node_index(g, i - g.off[0], j - g.off[1], k - g.off[2] + bx.zoff);
-      const int2 id = p.tab.ids[n];
-      int slot;
-      if (tag == id.x)
-        slot = 0;
-      else if (tag == id.y)
-        slot = 1;
-      else
-        continue;
-      const double* nf = nodeF + 6 * n + 3 * slot;
-      const double F0 = nf[0], F1 = nf[1], F2 = nf[2];
-      acc[0] += F0 * ff;
-      acc[1] += F1 * ff;
-      acc[2] += F2 * ff;
-      const double dx = (double)i - bx.xl[0];
-      const double dy = (double)j - bx.xl[1];
-      const double dz = (double)k - bx.xl[2];
-      acc[3] += (dy * F2 - dz * F1) * tf;
-      acc[4] += (dz * F0 - dx * F2) * tf;
-      acc[5] += (dx * F1 - dy * F0) * tf;
-      // 0.5*(a*b + a*b) is exactly a*b: doubling and halving are exact
-      acc[6] += (dx * F0) * tf;
-      acc[7] += (dy * F1) * tf;
-      acc[8] += (dz * F2) * tf;
-      acc[9] += 0.5 * (dy * F0 + dx * F1) * tf;
-      acc[10] += 0.5 * (dz * F0 + dx * F2) * tf;
-      acc[11] += 0.5 * (dz * F1 + dy * F2) * tf;
-    }
-  }
-  block_reduce_store(acc, p, ip);
-  copy_status(p);
 }
 
 // Error-free transformation: a + b = s + e exactly (Knuth's TwoSum; no
@@ -967,217 +881,296 @@ static __device__ __forceinline__ void two_sum(float a, float b, float& s, float
   e = (a - (s - bb)) + (b - bb);
 }
 
+// Twelve running sums of a lane (F, T, S before the unit factors).
+//
 // FP32 node forces (FP32 / FP16 / BF16 storage): per-node terms in FP32 (the
-// node forces carry FP32 precision), accumulated per particle in double-float
-// (hi + lo pairs combined with TwoSum, ~48-bit significand) on the FP32 pipe,
-// then the per-warp results summed in FP64.  (FP64 arithmetic runs at 1/64 of
-// the FP32 rate on this GPU.)  Issue- and latency-bound: 64 registers,
-// 64-thread blocks (16 per multiprocessor: the 2281 images of the 256^3
-// suspension run in one wave), two nodes'
-// loads in flight per thread, and only the nodes of each row that may lie
-// within rP visited (a sphere holds about half of its box), without the
-// divergence of testing every box node.  The order of the sums is fixed by
-// the image's box alone, so the results are reproducible bit for bit.
-constexpr int RED_U = 2;
-constexpr int RED32_THREADS = 64;  // FP32 reduction block
-__global__ void __launch_bounds__(RED32_THREADS, 16) reduce_f32_kernel(ReduceParams p) {
-  const int ip = blockIdx.x;
+// node forces carry FP32 precision), summed in double-float (hi + lo pairs
+// combined with TwoSum, ~48-bit significand) on the FP32 pipe.
+template <bool F64>
+struct Sums;
+template <>
+struct Sums<false> {
+  typedef float2 Pair;  // a partial sum, hi and lo
+  float hi[12], lo[12];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) hi[k] = lo[k] = 0.0f;
+  }
+  __device__ __forceinline__ void node(float F0, float F1, float F2, float dx, float dy, float dz) {
+    const float term[12] = {F0,
+                            F1,
+                            F2,
+                            dy * F2 - dz * F1,
+                            dz * F0 - dx * F2,
+                            dx * F1 - dy * F0,
+                            dx * F0,
+                            dy * F1,
+                            dz * F2,
+                            0.5f * (dy * F0 + dx * F1),
+                            0.5f * (dz * F0 + dx * F2),
+                            0.5f * (dz * F1 + dy * F2)};
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      float sv, e;
+      two_sum(hi[q], term[q], sv, e);
+      hi[q] = sv;
+      lo[q] += e;
+    }
+  }
+  static __device__ __forceinline__ Pair get(const Sums& s, int k) { return make_float2(s.hi[k], s.lo[k]); }
+  static __device__ __forceinline__ Pair zero() { return make_float2(0.0f, 0.0f); }
+  static __device__ __forceinline__ Pair pick(bool b, Pair x, Pair y) {
+    return make_float2(b ? x.x : y.x, b ? x.y : y.y);
+  }
+  static __device__ __forceinline__ Pair other(Pair x, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, x.x, o), __shfl_xor_sync(0xffffffffu, x.y, o));
+  }
+  static __device__ __forceinline__ Pair plus(Pair x, Pair y) {
+    float sv, e;
+    two_sum(x.x, y.x, sv, e);
+    return make_float2(sv, x.y + y.y + e);
+  }
+  static __device__ __forceinline__ double value(Pair x) { return (double)x.x + (double)x.y; }
+};
+// FP64 node forces: FP64 sums (the products in fused multiply-adds, the unit
+// factors once at the end: half the FP64 operations of the reference's
+// per-node expressions, on a pipe of 1.7 per clock and multiprocessor).
+template <>
+struct Sums<true> {
+  typedef double Pair;
+  double s[12];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) s[k] = 0.0;
+  }
+  __device__ __forceinline__ void node(double F0, double F1, double F2, double dx, double dy, double dz) {
+    s[0] += F0;
+    s[1] += F1;
+    s[2] += F2;
+    s[3] += __fma_rn(dy, F2, -(dz * F1));
+    s[4] += __fma_rn(dz, F0, -(dx * F2));
+    s[5] += __fma_rn(dx, F1, -(dy * F0));
+    s[6] = __fma_rn(dx, F0, s[6]);
+    s[7] = __fma_rn(dy, F1, s[7]);
+    s[8] = __fma_rn(dz, F2, s[8]);
+    s[9] += __fma_rn(dy, F0, dx * F1);  // twice the stresslet term, halved at the end
+    s[10] += __fma_rn(dz, F0, dx * F2);
+    s[11] += __fma_rn(dz, F1, dy * F2);
+  }
+  static __device__ __forceinline__ Pair get(const Sums& s, int k) { return s.s[k]; }
+  static __device__ __forceinline__ Pair zero() { return 0.0; }
+  static __device__ __forceinline__ Pair pick(bool b, Pair x, Pair y) { return b ? x : y; }
+  static __device__ __forceinline__ Pair other(Pair x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); }
+  static __device__ __forceinline__ Pair plus(Pair x, Pair y) { return x + y; }
+  static __device__ __forceinline__ double value(Pair x) { return x; }
+};
+
+// Per-image force, torque and stresslet (calculateHydrodynamicInteractions,
+// src/LBM_PSM_exchangeParticleData.cpp:172-244): the node forces of the
+// image's tag over its box.
+//
+// A solo image's tag can only sit on nodes within rP (eps > 0 from this
+// image), so each row is cut to the x-range that may lie within rP: an FP32
+// bound widened by 0.01 node, a superset (extra nodes fail the tag test).  The
+// rows of the box are taken in groups of 64, one warp a group, 32 rows at a
+// time, one per lane: the warp walks the nodes of their segments 32 at a time
+// (x fastest, consecutive lanes on consecutive nodes), a lane finding its
+// node's row by a binary search of the segments' offsets across the warp.  The
+// lanes' sums of a group are combined in a fixed tree, the groups' sums in
+// order, so the result depends on the image's box alone, however many warps
+// and blocks share its groups.
+//
+// C blocks (a cluster) share an image.  With many images one block of two
+// warps each keeps every multiprocessor busy (2260 images of diameter 12: one
+// wave); with few, eight blocks spread an image's groups over eight
+// multiprocessors, their sums meeting in the first block's shared memory (one
+// image of diameter 16: 45 us by one block).
+constexpr int RED_THREADS = 64;
+constexpr int RED_GROUP = 64;       // rows per group
+constexpr int RED_MAX_GROUPS = 32;  // groups whose sums are held at a time
+constexpr int RED_CLUSTER = 8;
+
+template <bool F64, int C>
+static __device__ __forceinline__ void reduce_image(const ReduceParams& p) {
+  typedef Sums<F64> S;
+  typedef typename S::Pair Pair;
+  constexpr int NW = RED_THREADS / 32;
+  // nodes per lane and round, loaded before any is summed (a lane sums its
+  // nodes in the same order whatever U)
+  constexpr int U = C == 1 ? (F64 ? 1 : 2) : (F64 ? 4 : 8);
+  __shared__ Pair part[RED_MAX_GROUPS][12];
+  const int ip = C == 1 ? (int)blockIdx.x : (int)blockIdx.x / C;
+  const int rank = C == 1 ? 0 : (int)blockIdx.x % C;
   const Geom& g = p.g;
   const int tag = p.tag[ip];
   const Img& bx = p.img[ip];  // box and centre from the map's image record
   const int wx = bx.qhi[0] - bx.qlo[0], wy = bx.qhi[1] - bx.qlo[1], wz = bx.qhi[2] - bx.qlo[2];
-  float hi[12], lo[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) hi[k] = lo[k] = 0.0f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (wx > 0 && wy > 0 && wz > 0) {
-    const int xi[3] = {bx.xi[0], bx.xi[1], bx.xi[2]};  // xl = xi + xf exactly
-    const float xf[3] = {bx.xf[0], bx.xf[1], bx.xf[2]};
-    const float* nodeF = static_cast<const float*>(p.tab.nodeF);
-    const int R = wy * wz;  // x-rows of the box
-    const FastDiv fy = make_fastdiv((unsigned)wy);
-    // A solo image's tag can only sit on nodes within rP (eps > 0 from this
-    // image), so each row is cut to the x-range that may lie within rP: an
-    // FP32 bound widened by 0.01 node, a superset (extra nodes fail the tag
-    // test).  Each warp takes 32 rows at a time, one per lane, and walks the
-    // nodes of their segments 32 at a time (x fastest, consecutive lanes on
-    // consecutive nodes); a lane finds its node's row by a binary search of
-    // the segments' offsets across the warp.
-    const float rem0 = bx.rP2f * 1.0001f + 0.01f;
-    for (int r0 = warp * 32; r0 < R; r0 += RED32_THREADS) {
-      const int r = r0 + lane;
-      int xa = bx.qlo[0], len = 0, j = 0, k = 0;
-      if (r < R) {
-        const int q = (int)fast_div((unsigned)r, fy);
-        j = bx.qlo[1] + r - q * wy;
-        k = bx.qlo[2] + q;
-        int xb = bx.qhi[0];
-        if (bx.solo) {
-          const float dy = small_int_to_float(j - xi[1]) - xf[1];
-          const float dz = small_int_to_float(k - xi[2]) - xf[2];
-          const float rem = rem0 - dy * dy - dz * dz;
-          if (rem < 0.0f) {
-            xb = xa;
-          } else {
-            const float h = sqrtf(rem) + 0.01f;
-            xa = max(xa, xi[0] + (int)ceilf(xf[0] - h));
-            xb = min(xb, xi[0] + (int)floorf(xf[0] + h) + 1);
+  const int R = wx > 0 && wy > 0 && wz > 0 ? wy * wz : 0;  // x-rows of the box
+  const int G = (R + RED_GROUP - 1) / RED_GROUP;
+  const FastDiv fy = make_fastdiv((unsigned)max(wy, 1));
+  const int xi[3] = {bx.xi[0], bx.xi[1], bx.xi[2]};  // xl = xi + xf exactly
+  const float xf[3] = {bx.xf[0], bx.xf[1], bx.xf[2]};
+  const double xl0 = F64 ? bx.xl[0] : 0.0;
+  const float rem0 = bx.rP2f * 1.0001f + 0.01f;
+  Pair total = S::zero();  // thread k < 12 of the first block: sum k
+  for (int g0 = 0; g0 < G || g0 == 0; g0 += RED_MAX_GROUPS) {
+    const int gend = min(G, g0 + RED_MAX_GROUPS);
+    for (int gi = g0 + rank * NW + warp; gi < gend; gi += C * NW) {
+      S acc;
+      acc.clear();
+#pragma unroll 1
+      for (int r0 = gi * RED_GROUP; r0 < min(R, (gi + 1) * RED_GROUP); r0 += 32) {
+        const int r = r0 + lane;
+        int xa = bx.qlo[0], len = 0, j = 0, k = 0;
+        float fdy = 0.0f, fdz = 0.0f;
+        double ddy = 0.0, ddz = 0.0;
+        if (r < R) {
+          const int q = (int)fast_div((unsigned)r, fy);
+          j = bx.qlo[1] + r - q * wy;
+          k = bx.qlo[2] + q;
+          int xb = bx.qhi[0];
+          fdy = small_int_to_float(j - xi[1]) - xf[1];
+          fdz = small_int_to_float(k - xi[2]) - xf[2];
+          if (bx.solo) {
+            const float rem = rem0 - fdy * fdy - fdz * fdz;
+            if (rem < 0.0f) {
+              xb = xa;
+            } else {
+              const float h = sqrtf(rem) + 0.01f;
+              xa = max(xa, xi[0] + (int)ceilf(xf[0] - h));
+              xb = min(xb, xi[0] + (int)floorf(xf[0] + h) + 1);
+            }
+          }
+          len = max(xb - xa, 0);
+          if (F64) {
+            ddy = small_int_to_double(j) - bx.xl[1];
+            ddz = small_int_to_double(k) - bx.xl[2];
           }
         }
-        len = max(xb - xa, 0);
-      }
-      int incl = len;
+        int incl = len;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const int excl = incl - len;
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      // RED_U nodes per lane and round, loaded before any is summed
-      for (int base = 0; base < total; base += RED_U * 32) {
-        int2 id[RED_U];
-        float2 f01[RED_U], f23[RED_U], f45[RED_U];
-        float dx[RED_U], dy[RED_U], dz[RED_U];
-        bool ok[RED_U];
-#pragma unroll
-        for (int u = 0; u < RED_U; ++u) {
-          const int t = base + u * 32 + lane;
-          // the row holding node t: the last lane whose offset is <= t (a
-          // row of length 0 shares its offset with the next row)
-          int l = 0;
-#pragma unroll
-          for (int st = 16; st >= 1; st >>= 1)
-            if (__shfl_sync(0xffffffffu, excl, l + st) <= t) l += st;
-          const int ra = __shfl_sync(0xffffffffu, xa, l);
-          const int re = __shfl_sync(0xffffffffu, excl, l);
-          const int jj = __shfl_sync(0xffffffffu, j, l);
-          const int kk = __shfl_sync(0xffffffffu, k, l);
-          const int i = ra + t - re;
-          ok[u] = t < total;
-          id[u] = make_int2(0, 0);
-          f01[u] = f23[u] = f45[u] = make_float2(0.f, 0.f);
-          dx[u] = small_int_to_float(i - xi[0]) - xf[0];
-          dy[u] = small_int_to_float(jj - xi[1]) - xf[1];
-          dz[u] = small_int_to_float(kk - xi[2]) - xf[2];
-          if (ok[u]) {
-            const long long n = node_index(g, i - g.off[0], jj - g.off[1], kk - g.off[2] + bx.zoff);
-            // both slots' forces are loaded with the ids (no second dependent load)
-            id[u] = p.tab.ids[n];
-            const float2* nf2 = reinterpret_cast<const float2*>(nodeF + 6 * n);
-            f01[u] = nf2[0];
-            f23[u] = nf2[1];
-            f45[u] = nf2[2];
-          }
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
         }
+        const int excl = incl - len;
+        const int count = __shfl_sync(0xffffffffu, incl, 31);
+        for (int base = 0; base < count; base += U * 32) {
+          int2 id[U];
+          float2 f01[U], f23[U], f45[U];
+          double d0[U], d1[U], d2[U], d3[U], d4[U], d5[U];
+          float dx[U], dy[U], dz[U];
+          double ex[U], ey[U], ez[U];
+          bool ok[U];
 #pragma unroll
-        for (int u = 0; u < RED_U; ++u) {
-          if (!ok[u]) continue;
-          float F0, F1, F2;
-          if (tag == id[u].x) {
-            F0 = f01[u].x;
-            F1 = f01[u].y;
-            F2 = f23[u].x;
-          } else if (tag == id[u].y) {
-            F0 = f23[u].y;
-            F1 = f45[u].x;
-            F2 = f45[u].y;
-          } else {
-            continue;
+          for (int u = 0; u < U; ++u) {
+            const int t = base + u * 32 + lane;
+            // the row holding node t: the last lane whose offset is <= t (a
+            // row of length 0 shares its offset with the next row)
+            int l = 0;
+#pragma unroll
+            for (int st = 16; st >= 1; st >>= 1)
+              if (__shfl_sync(0xffffffffu, excl, l + st) <= t) l += st;
+            const int ra = __shfl_sync(0xffffffffu, xa, l);
+            const int re = __shfl_sync(0xffffffffu, excl, l);
+            const int jj = __shfl_sync(0xffffffffu, j, l);
+            const int kk = __shfl_sync(0xffffffffu, k, l);
+            const int i = ra + t - re;
+            ok[u] = t < count;
+            id[u] = make_int2(0, 0);
+            if (F64) {
+              ey[u] = __shfl_sync(0xffffffffu, ddy, l);
+              ez[u] = __shfl_sync(0xffffffffu, ddz, l);
+            } else {
+              f01[u] = f23[u] = f45[u] = make_float2(0.f, 0.f);
+              dx[u] = small_int_to_float(i - xi[0]) - xf[0];
+              dy[u] = small_int_to_float(jj - xi[1]) - xf[1];
+              dz[u] = small_int_to_float(kk - xi[2]) - xf[2];
+            }
+            if (ok[u]) {
+              const long long n = node_index(g, i - g.off[0], jj - g.off[1], kk - g.off[2] + bx.zoff);
+              // both slots' forces are loaded with the ids (no second dependent load)
+              id[u] = p.tab.ids[n];
+              if (F64) {
+                const double2* nf2 = reinterpret_cast<const double2*>(static_cast<const double*>(p.tab.nodeF) + 6 * n);
+                const double2 a = nf2[0], b = nf2[1], c = nf2[2];
+                d0[u] = a.x; d1[u] = a.y; d2[u] = b.x;
+                d3[u] = b.y; d4[u] = c.x; d5[u] = c.y;
+                ex[u] = small_int_to_double(i) - xl0;
+              } else {
+                const float2* nf2 = reinterpret_cast<const float2*>(static_cast<const float*>(p.tab.nodeF) + 6 * n);
+                f01[u] = nf2[0];
+                f23[u] = nf2[1];
+                f45[u] = nf2[2];
+              }
+            }
           }
-          const float term[12] = {F0,
-                                  F1,
-                                  F2,
-                                  dy[u] * F2 - dz[u] * F1,
-                                  dz[u] * F0 - dx[u] * F2,
-                                  dx[u] * F1 - dy[u] * F0,
-                                  dx[u] * F0,
-                                  dy[u] * F1,
-                                  dz[u] * F2,
-                                  0.5f * (dy[u] * F0 + dx[u] * F1),
-                                  0.5f * (dz[u] * F0 + dx[u] * F2),
-                                  0.5f * (dz[u] * F1 + dy[u] * F2)};
 #pragma unroll
-          for (int q = 0; q < 12; ++q) {
-            float sv, e;
-            two_sum(hi[q], term[q], sv, e);
-            hi[q] = sv;
-            lo[q] += e;
+          for (int u = 0; u < U; ++u) {
+            if (!ok[u]) continue;
+            const bool one = tag == id[u].x, two = tag == id[u].y;
+            if (!one && !two) continue;
+            if constexpr (F64)
+              acc.node(one ? d0[u] : d3[u], one ? d1[u] : d4[u], one ? d2[u] : d5[u], ex[u], ey[u], ez[u]);
+            else
+              acc.node(one ? f01[u].x : f23[u].y, one ? f01[u].y : f45[u].x, one ? f23[u].x : f45[u].y,
+                       dx[u], dy[u], dz[u]);
           }
         }
       }
+      // fixed-order reduction within the warp: the first two levels halve the
+      // terms each lane carries (12 -> 6 -> 3, partners keeping complementary
+      // halves), the last three are a butterfly on three terms
+      const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+      Pair h6[6], h3[3];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const Pair x = S::get(acc, k), y = S::get(acc, k + 6);
+        h6[k] = S::plus(S::pick(up16, y, x), S::other(S::pick(up16, x, y), 16));
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        h3[k] = S::plus(S::pick(up8, h6[k + 3], h6[k]), S::other(S::pick(up8, h6[k], h6[k + 3]), 8));
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) h3[k] = S::plus(h3[k], S::other(h3[k], o));
+      if ((lane & 7) == 0) {  // lanes 0, 8, 16, 24 hold terms 0-2, 3-5, 6-8, 9-11
+        const int q0 = (up16 ? 6 : 0) + (up8 ? 3 : 0);
+        Pair* dst = &part[gi - g0][q0];
+        if (C > 1) dst = cooperative_groups::this_cluster().map_shared_rank(dst, 0);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dst[k] = h3[k];
+      }
+    }
+    if (C > 1)
+      cooperative_groups::this_cluster().sync();
+    else
+      __syncthreads();
+    if (rank == 0 && threadIdx.x < 12)
+      for (int k = 0; k < gend - g0; ++k) total = S::plus(total, part[k][threadIdx.x]);
+    if (G > RED_MAX_GROUPS) {  // the sums are read before the next groups' arrive
+      if (C > 1)
+        cooperative_groups::this_cluster().sync();
+      else
+        __syncthreads();
     }
   }
-  // fixed-order double-float reduction within the warp: the first two levels
-  // halve the terms each lane carries (12 -> 6 -> 3, partners keeping
-  // complementary halves), the last three are a butterfly on three terms
-  const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
-  float h6[6], l6[6], h3[3], l3[3];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const float sh = up16 ? hi[k] : hi[k + 6], sl = up16 ? lo[k] : lo[k + 6];
-    const float mh = up16 ? hi[k + 6] : hi[k], ml = up16 ? lo[k + 6] : lo[k];
-    const float rh = __shfl_xor_sync(0xffffffffu, sh, 16);
-    const float rl = __shfl_xor_sync(0xffffffffu, sl, 16);
-    float sv, e;
-    two_sum(mh, rh, sv, e);
-    h6[k] = sv;
-    l6[k] = ml + rl + e;
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float sh = up8 ? h6[k] : h6[k + 3], sl = up8 ? l6[k] : l6[k + 3];
-    const float mh = up8 ? h6[k + 3] : h6[k], ml = up8 ? l6[k + 3] : l6[k];
-    const float rh = __shfl_xor_sync(0xffffffffu, sh, 8);
-    const float rl = __shfl_xor_sync(0xffffffffu, sl, 8);
-    float sv, e;
-    two_sum(mh, rh, sv, e);
-    h3[k] = sv;
-    l3[k] = ml + rl + e;
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      const float h2 = __shfl_xor_sync(0xffffffffu, h3[k], o);
-      const float l2 = __shfl_xor_sync(0xffffffffu, l3[k], o);
-      float sv, e;
-      two_sum(h3[k], h2, sv, e);
-      h3[k] = sv;
-      l3[k] = l3[k] + l2 + e;
-    }
-  }
-  // warps in index order, still in double-float; one FP64 sum per term
-  __shared__ float part_hi[RED32_THREADS / 32][12], part_lo[RED32_THREADS / 32][12];
-  if ((lane & 7) == 0) {  // lanes 0, 8, 16, 24 hold terms 0-2, 3-5, 6-8, 9-11
-    const int q0 = (up16 ? 6 : 0) + (up8 ? 3 : 0);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      part_hi[warp][q0 + k] = h3[k];
-      part_lo[warp][q0 + k] = l3[k];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 12) {
+  if (rank == 0 && threadIdx.x < 12) {
     const int q = threadIdx.x;
-    float sh = 0.0f, sl = 0.0f;
-    for (int w = 0; w < RED32_THREADS / 32; ++w) {
-      float sv, e;
-      two_sum(sh, part_hi[w][q], sv, e);
-      sh = sv;
-      sl = sl + part_lo[w][q] + e;
-    }
-    const double sum = (double)sh + (double)sl;
+    const double sum = S::value(total);
+    const BoxParams& bp = p.box[bx.bidx];
     if (q < 3) {
-      const double v = sum * p.box[bx.bidx].forceFactor;
+      const double v = sum * bp.forceFactor;
       p.fh[3 * ip + q] = v;
       if (p.fh2) p.fh2[3 * ip + q] = v;
     } else if (q < 6) {
-      const double v = sum * p.box[bx.bidx].torqueFactor;
+      const double v = sum * bp.torqueFactor;
       p.th[3 * ip + (q - 3)] = v;
       if (p.th2) p.th2[3 * ip + (q - 3)] = v;
     } else {
-      const double v = -(sum * p.box[bx.bidx].torqueFactor);
+      const double v = -((F64 && q >= 9 ? 0.5 * sum : sum) * bp.torqueFactor);
       p.S[6 * ip + (q - 6)] = v;
       if (p.S2) p.S2[6 * ip + (q - 6)] = v;
     }
@@ -1185,18 +1178,44 @@ __global__ void __launch_bounds__(RED32_THREADS, 16) reduce_f32_kernel(ReducePar
   copy_status(p);
 }
 
+__global__ void __launch_bounds__(RED_THREADS, 16) reduce_f32_kernel(ReduceParams p) {
+  reduce_image<false, 1>(p);
+}
+__global__ void __launch_bounds__(RED_THREADS) reduce_f64_kernel(ReduceParams p) {
+  reduce_image<true, 1>(p);
+}
+__global__ void __launch_bounds__(RED_THREADS) __cluster_dims__(RED_CLUSTER, 1, 1)
+    reduce_f32_few_kernel(ReduceParams p) {
+  reduce_image<false, RED_CLUSTER>(p);
+}
+__global__ void __launch_bounds__(RED_THREADS) __cluster_dims__(RED_CLUSTER, 1, 1)
+    reduce_f64_few_kernel(ReduceParams p) {
+  reduce_image<true, RED_CLUSTER>(p);
+}
+
 cudaError_t launch_reduce(const ReduceParams& p, cudaStream_t st) {
   if (p.n <= 0) return cudaSuccess;
-  if (p.nodeF_is_double)
-    reduce_f64_kernel<<<p.n, RED_THREADS, 0, st>>>(p);
-  else
-    reduce_f32_kernel<<<p.n, RED32_THREADS, 0, st>>>(p);
+  const bool few = few_images(p.n, p.sm_count);
+  const unsigned grid = (unsigned)p.n * (few ? RED_CLUSTER : 1);
+  if (p.nodeF_is_double) {
+    if (few)
+      reduce_f64_few_kernel<<<grid, RED_THREADS, 0, st>>>(p);
+    else
+      reduce_f64_kernel<<<grid, RED_THREADS, 0, st>>>(p);
+  } else {
+    if (few)
+      reduce_f32_few_kernel<<<grid, RED_THREADS, 0, st>>>(p);
+    else
+      reduce_f32_kernel<<<grid, RED_THREADS, 0, st>>>(p);
+  }
   return cudaGetLastError();
 }
 
 // the kernels whose parameters a replayed device-step graph updates per call
 const void* img_prep_fn() { return (const void*)img_prep_kernel; }
-const void* reduce_fn(int nodeF_is_double) {
+const void* reduce_fn(int nodeF_is_double, int n, int sm_count) {
+  if (few_images(n, sm_count))
+    return nodeF_is_double ? (const void*)reduce_f64_few_kernel : (const void*)reduce_f32_few_kernel;
   return nodeF_is_double ? (const void*)reduce_f64_kernel : (const void*)reduce_f32_kernel;
 }
 
