@@ -186,6 +186,8 @@ __device__ __forceinline__ void node_slots(const AdjParams& p, long long n, Node
   for (int k = 0; k < 2; ++k)
 #pragma unroll
     for (int c = 0; c < 3; ++c) s.us[k][c] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) s.w.B[k] = s.w.dBde[k][0] = s.w.dBde[k][1] = s.w.dBdtau[k] = 0.0;
   if (!flag && !band) return;
   int2 id = make_int2(0, 0);
   double2 e = make_double2(0.0, 0.0);
