@@ -228,8 +228,10 @@ int lbmpsm_host_direct(const lbmpsm_handle* h);
 /* Run nsteps coupling steps with the particle images already on the device
  * (as last passed to lbmpsm_step or lbmpsm_step_device), fixed in place,
  * each step followed by the boundary condition when one is set.  The step
- * sequence is captured once into a CUDA graph and replayed.  The forces of
- * each step land in the handle's own buffers (read with lbmpsm_read_forces). */
+ * sequence is captured once into a CUDA graph and replayed.  A call of several
+ * steps waits after its first ones to see whether the particle table has
+ * settled; from then on its steps run without the map.  The forces of each
+ * step land in the handle's own buffers (read with lbmpsm_read_forces). */
 int lbmpsm_run_fixed(lbmpsm_handle* h, int nsteps);
 /* Copy the per-image outputs of the last step to host memory. */
 int lbmpsm_read_forces(lbmpsm_handle* h, int n, double* fh, double* th, double* stresslet);

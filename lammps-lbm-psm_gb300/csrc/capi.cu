@@ -68,7 +68,7 @@ struct lbmpsm_handle {
   int4* d_lrec = nullptr;  // records per cell-list entry (3 int4 each)
   unsigned short* d_sfcode = nullptr;  // solid-fraction codes of (image, box node) pairs
   long long sf_cap = 0;
-  unsigned long long* d_pair_total = nullptr;  // [0] list pairs, [1] codes, [2] shell nodes
+  unsigned long long* d_pair_total = nullptr;  // [0] list pairs, [1] codes, [2] shell nodes, [3] an id changed
   int4* d_shell = nullptr;  // shell nodes of the solid-fraction map (sf_cap entries)
   int sm_count = 1;
   int* d_status = nullptr;
@@ -80,6 +80,8 @@ struct lbmpsm_handle {
   int last_n = 0;
   // graphs of one step for each parity (map + collide + reduce + bc)
   cudaGraphExec_t gexec[2]{nullptr, nullptr};
+  // the same without the map, for steps on a settled table (map_settled)
+  cudaGraphExec_t sexec[2]{nullptr, nullptr};
   // graphs of one host-pointer step for each parity (upload of the staged
   // images, map + collide + reduce, download of the outputs and status word)
   cudaGraphExec_t hexec[2]{nullptr, nullptr};
@@ -294,11 +296,12 @@ void free_particles(lbmpsm_handle* h) {
 }
 
 void drop_run_graphs(lbmpsm_handle* h) {
-  for (int k = 0; k < 2; ++k)
-    if (h->gexec[k]) {
-      cudaGraphExecDestroy(h->gexec[k]);
-      h->gexec[k] = nullptr;
-    }
+  for (cudaGraphExec_t* ex : {h->gexec, h->sexec})
+    for (int k = 0; k < 2; ++k)
+      if (ex[k]) {
+        cudaGraphExecDestroy(ex[k]);
+        ex[k] = nullptr;
+      }
   h->graph_n = -1;
 }
 
@@ -515,11 +518,12 @@ int enqueue_bc(lbmpsm_handle* h, cudaStream_t st);
 // also the boundary faces after the collide.  The faces touch only the
 // populations, which neither the reduction nor the next step's map reads,
 // so with images the face kernel runs on the auxiliary stream beside the
-// reduction.
-int enqueue_step(lbmpsm_handle* h, int n, bool bc = false);
+// reduction.  Without map: on a settled table (map_settled).
+// held: the images are held in place, the map notes whether it changes an id.
+int enqueue_step(lbmpsm_handle* h, int n, bool bc = false, bool map = true, bool held = false);
 
 // The particle map of a step with n images (nothing without images).
-int enqueue_map(lbmpsm_handle* h, int n) {
+int enqueue_map(lbmpsm_handle* h, int n, bool held = false) {
   // image block layout: x | v | omega (3n each) | radius (n)
   const int* tag = h->d_tag;
   const double* x = h->d_xvw;
@@ -565,6 +569,7 @@ int enqueue_map(lbmpsm_handle* h, int n) {
     m.lrec = h->d_lrec;
     m.list_cap = h->list_cap;
     m.pair_total = h->d_pair_total;
+    m.changed = held ? h->d_pair_total + 3 : nullptr;
     m.sfcode = h->d_sfcode;
     m.sf_cap = h->sf_cap;
     m.sf_value = h->d_sf_value;
@@ -623,8 +628,8 @@ int enqueue_post(lbmpsm_handle* h, int n, bool bc) {
   return LBMPSM_OK;
 }
 
-int enqueue_step(lbmpsm_handle* h, int n, bool bc) {
-  int rc = enqueue_map(h, n);
+int enqueue_step(lbmpsm_handle* h, int n, bool bc, bool map, bool held) {
+  int rc = map ? enqueue_map(h, n, held) : LBMPSM_OK;
   if (!rc) rc = collide(h);
   if (!rc) rc = enqueue_post(h, n, bc);
   return rc;
@@ -650,6 +655,24 @@ int enqueue_bc(lbmpsm_handle* h, cudaStream_t st) {
   CUDA_TRY(h, e);
   return LBMPSM_OK;
 }
+
+// Whether the last map (of a held step) left every slot id as it found it, at every image of
+// every node.  Each update depends on the images and on the node's ids alone,
+// so another map of the same images would take the same ids through the same
+// updates and write the same records: within a run of steps with images held
+// in place the map need not run again (it is 110 of 175 us of a step of one
+// sphere in 128^3, 210 of 640 us of the 256^3 suspension's).  Waits for the
+// stream.
+int map_settled(lbmpsm_handle* h, cudaStream_t st, bool& settled) {
+  unsigned long long changed = 1;
+  CUDA_TRY(h, cudaMemcpyAsync(&changed, h->d_pair_total + 3, sizeof(changed), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(h, cudaStreamSynchronize(st));
+  settled = changed == 0;
+  return LBMPSM_OK;
+}
+// Steps of a run after which it is asked (a table that particles have just
+// moved over settles with the second or third map).
+bool ask_settled(int step) { return step >= 1 && step <= 3; }
 
 int read_status(lbmpsm_handle* h) {
   int st = 0;
@@ -1520,13 +1543,22 @@ int lbmpsm_run_fixed(lbmpsm_handle* h, int nsteps) {
     if (rc) return rc;
     --nsteps;
   }
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CUDA_TRY(h, cudaStreamIsCapturing(h->stream, &cs));
+  const bool may_settle = n > 0 && cs == cudaStreamCaptureStatusNone;
+  bool settled = false;
   for (int s = 0; s < nsteps; ++s) {
     const int par = (int)(h->t & 1);
-    if (!h->gexec[par]) {
+    if (may_settle && !settled && ask_settled(s) && nsteps - s >= 4) {
+      const int rc = map_settled(h, h->stream, settled);
+      if (rc) return rc;
+    }
+    cudaGraphExec_t* const exec = settled ? h->sexec : h->gexec;
+    if (!exec[par]) {
       cudaGraph_t graph = nullptr;
       CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
       const long long t0 = h->t;
-      int rc = enqueue_step(h, n, use_bc);
+      int rc = enqueue_step(h, n, use_bc, !settled, true);
       cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
       h->t = t0;  // captured, not run
       if (rc) {
@@ -1534,13 +1566,13 @@ int lbmpsm_run_fixed(lbmpsm_handle* h, int nsteps) {
         return rc;
       }
       CUDA_TRY(h, ce);
-      cudaError_t ie = cudaGraphInstantiate(&h->gexec[par], graph, 0);
+      cudaError_t ie = cudaGraphInstantiate(&exec[par], graph, 0);
       cudaGraphDestroy(graph);
       CUDA_TRY(h, ie);
       h->graph_n = n;
       h->graph_bc = use_bc;
     }
-    CUDA_TRY(h, cudaGraphLaunch(h->gexec[par], h->stream));
+    CUDA_TRY(h, cudaGraphLaunch(exec[par], h->stream));
     h->t += 1;
   }
   return LBMPSM_OK;
@@ -1640,8 +1672,9 @@ extern "C" int lbmpsm_export_fields_static(lbmpsm_handle* h, int as_double, doub
 // lbmpsm_tangent_drag).
 //
 // Both calls run nsteps ordinary coupling steps with one fixed set of
-// particle images -- the same map / collide / reduce launches as nsteps
-// lbmpsm_step calls, so the lattice ends where those calls would leave it and
+// particle images -- the map / collide / reduce launches of nsteps lbmpsm_step
+// calls (without the maps of a settled table), so the lattice ends where those
+// calls would leave it and
 // J is the average of the forces they would return -- and differentiate
 //   J = 1/M sum_{t=t0..t1} sum_images d . F_image(t),   M = t1 - t0 + 1,
 // with respect to tau, Fext and the image centres (kernels in adjoint.cu).
@@ -1853,14 +1886,19 @@ int lbmpsm_adjoint_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
 
   // forward pass: the ordinary steps, a checkpoint before every K-th
   const long long ts = h->t;
+  bool settled = false;
   for (int t = 1; t <= T; ++t) {
     if ((t - 1) % K == 0)
       CUDA_TRY(h, cudaMemcpyAsync(ckpt[(size_t)((t - 1) / K)], h->f, state,
                                   cudaMemcpyDeviceToDevice, h->stream));
-    rc = enqueue_step(h, n);
+    rc = enqueue_step(h, n, false, !settled, true);
     if (rc) return rc;
     if (t == 1) {
       rc = adj_entries(h, an, n, centre_step);
+      if (rc) return rc;
+    }
+    if (n > 0 && !settled && ask_settled(t) && t < T) {
+      rc = map_settled(h, h->stream, settled);
       if (rc) return rc;
     }
     if (n > 0)
@@ -1959,6 +1997,7 @@ int lbmpsm_tangent_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   const double cwin = h->forceFactor / (double)(t1 - t0 + 1);
   const long long ts = h->t;
   int cur = 0;
+  bool settled = false;
   for (int t = 1; t <= T; ++t) {
     // the tangent step reads the state before this step's collide; the table
     // it needs exists after the first map, so step 1 runs from a copy
@@ -1972,8 +2011,12 @@ int lbmpsm_tangent_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
       CUDA_TRY(h, launch_adj_step(p, 1, h->stream));
       cur ^= 1;
     }
-    rc = enqueue_step(h, n);
+    rc = enqueue_step(h, n, false, !settled, true);
     if (rc) return rc;
+    if (n > 0 && !settled && ask_settled(t) && t < T) {
+      rc = map_settled(h, h->stream, settled);
+      if (rc) return rc;
+    }
     if (t == 1) {
       rc = adj_entries(h, an, n, centre_step);
       if (rc) return rc;
@@ -2023,6 +2066,7 @@ struct lbmpsm_group {
   cudaEvent_t fork = nullptr, done = nullptr, fork2 = nullptr;
   std::vector<cudaEvent_t> join, join2;
   cudaGraphExec_t gexec[2]{nullptr, nullptr};
+  cudaGraphExec_t sexec[2]{nullptr, nullptr};  // without the maps, on settled tables
   std::vector<long long> gen;  // members' graph generations the graphs were captured at
   std::vector<int> cap_n, cap_bc;
   std::string err;
@@ -2055,11 +2099,15 @@ int gfail(lbmpsm_group* g, int code, const std::string& msg) {
   } while (0)
 
 void group_drop(lbmpsm_group* g) {
-  for (int k = 0; k < 2; ++k)
-    if (g->gexec[k]) {
-      cudaGraphExecDestroy(g->gexec[k]);
-      g->gexec[k] = nullptr;
-    }
+  for (cudaGraphExec_t* ex : {g->gexec, g->sexec})
+    for (int k = 0; k < 2; ++k)
+      if (ex[k]) {
+        cudaGraphExecDestroy(ex[k]);
+        ex[k] = nullptr;
+      }
+}
+bool group_captured(const lbmpsm_group* g) {
+  return g->gexec[0] || g->gexec[1] || g->sexec[0] || g->sexec[1];
 }
 
 // Whether the members' collides run as one launch, and if so its member
@@ -2115,17 +2163,28 @@ int group_plan_collide(lbmpsm_group* g) {
   return LBMPSM_OK;
 }
 
-// Capture the graph of one step of every member for parity par.
-int group_capture(lbmpsm_group* g, int par) {
+// Capture the graph of one step of every member for parity par, with the
+// members' maps or (on settled tables) without.
+int group_capture(lbmpsm_group* g, int par, bool map) {
   const size_t m = g->hs.size();
   cudaGraph_t graph = nullptr;
   std::vector<long long> t0(m);
-  for (size_t i = 0; i < m; ++i) t0[i] = g->hs[i]->t;
-  if (!g->gexec[par ^ 1]) {  // planned once for both parities' graphs
-    const int prc = group_plan_collide(g);
-    if (prc) return prc;
+  for (size_t i = 0; i < m; ++i) {
+    t0[i] = g->hs[i]->t;
+    if ((int)(t0[i] & 1) != par) g->hs[i]->t += 1;  // captured ahead of its step
   }
-  GROUP_TRY(g, cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
+  if (!group_captured(g)) {  // planned once for all graphs
+    const int prc = group_plan_collide(g);
+    if (prc) {
+      for (size_t i = 0; i < m; ++i) g->hs[i]->t = t0[i];
+      return prc;
+    }
+  }
+  const cudaError_t be = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal);
+  if (be != cudaSuccess) {
+    for (size_t i = 0; i < m; ++i) g->hs[i]->t = t0[i];
+    GROUP_TRY(g, be);
+  }
   int rc = LBMPSM_OK;
   cudaError_t ce = cudaEventRecord(g->fork, g->stream);
   if (!g->fused) {
@@ -2134,7 +2193,7 @@ int group_capture(lbmpsm_group* g, int par) {
       lbmpsm_handle* h = g->hs[i];
       ce = cudaStreamWaitEvent(h->stream, g->fork, 0);
       if (ce != cudaSuccess) break;
-      rc = enqueue_step(h, h->last_n, true);
+      rc = enqueue_step(h, h->last_n, true, map, true);
       if (rc) rc = gfail(g, rc, h->err);
       if (!rc) ce = cudaEventRecord(g->join[i], h->stream);
       if (!rc && ce == cudaSuccess) ce = cudaStreamWaitEvent(g->stream, g->join[i], 0);
@@ -2146,7 +2205,7 @@ int group_capture(lbmpsm_group* g, int par) {
       lbmpsm_handle* h = g->hs[i];
       ce = cudaStreamWaitEvent(h->stream, g->fork, 0);
       if (ce != cudaSuccess) break;
-      rc = enqueue_map(h, h->last_n);
+      if (map) rc = enqueue_map(h, h->last_n, true);
       if (rc) rc = gfail(g, rc, h->err);
       if (!rc) ce = cudaEventRecord(g->join[i], h->stream);
       if (!rc && ce == cudaSuccess) ce = cudaStreamWaitEvent(g->stream, g->join[i], 0);
@@ -2175,7 +2234,7 @@ int group_capture(lbmpsm_group* g, int par) {
     GROUP_TRY(g, ce);
     GROUP_TRY(g, ee);
   }
-  cudaError_t ie = cudaGraphInstantiate(&g->gexec[par], graph, 0);
+  cudaError_t ie = cudaGraphInstantiate(map ? &g->gexec[par] : &g->sexec[par], graph, 0);
   cudaGraphDestroy(graph);
   GROUP_TRY(g, ie);
   g->gen.resize(m);
@@ -2191,13 +2250,14 @@ int group_capture(lbmpsm_group* g, int par) {
 
 // One step of the group: its graph for the members' parity (captured on
 // first use), launched on the group's stream.
-int group_step(lbmpsm_group* g) {
+int group_step(lbmpsm_group* g, bool map) {
   const int par = (int)(g->hs[0]->t & 1);
-  if (!g->gexec[par]) {
-    const int rc = group_capture(g, par);
+  cudaGraphExec_t* const exec = map ? g->gexec : g->sexec;
+  if (!exec[par]) {
+    const int rc = group_capture(g, par, map);
     if (rc) return rc;
   }
-  GROUP_TRY(g, cudaGraphLaunch(g->gexec[par], g->stream));
+  GROUP_TRY(g, cudaGraphLaunch(exec[par], g->stream));
   for (lbmpsm_handle* h : g->hs) h->t += 1;
   return LBMPSM_OK;
 }
@@ -2271,7 +2331,7 @@ int lbmpsm_group_tune_ms(const lbmpsm_group* g, float* ms) {
 }
 
 int lbmpsm_group_collide_launches(const lbmpsm_group* g) {
-  if (!g || (!g->gexec[0] && !g->gexec[1])) return -1;
+  if (!g || !group_captured(g)) return -1;
   return g->fused ? 1 : (int)g->hs.size();
 }
 
@@ -2302,6 +2362,26 @@ int lbmpsm_group_run_fixed(lbmpsm_group* g, int nsteps) {
     GROUP_TRY(g, cudaEventRecord(g->join[i], g->hs[i]->stream));
     GROUP_TRY(g, cudaStreamWaitEvent(g->stream, g->join[i], 0));
   }
+  // one step; after the first ones, whether every member's table is settled
+  // (map_settled: from then on the steps run without the maps)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  GROUP_TRY(g, cudaStreamIsCapturing(g->stream, &cs));
+  bool settled = false;
+  int done = 0;
+  auto step = [&]() -> int {
+    if (!settled && cs == cudaStreamCaptureStatusNone && ask_settled(done) && nsteps >= 4) {
+      settled = true;
+      for (size_t i = 0; settled && i < m; ++i) {
+        if (g->hs[i]->last_n == 0) continue;
+        const int rc = map_settled(g->hs[i], g->stream, settled);
+        if (rc) return gfail(g, rc, g->hs[i]->err);
+      }
+    }
+    const int rc = group_step(g, !settled);
+    ++done;
+    --nsteps;
+    return rc;
+  };
   // the group's tuner: with at least 8 steps to run and members that qualify
   // for one collide launch, time two steps of each plan (after two untimed
   // steps that capture its graphs) and keep the faster
@@ -2312,12 +2392,17 @@ int lbmpsm_group_run_fixed(lbmpsm_group* g, int nsteps) {
       group_drop(g);
       g->plan_pref = plan;
       for (int k = 0; k < 2; ++k) {
-        const int rc = group_step(g);
+        const int rc = step();
+        if (rc) return rc;
+      }
+      for (int par = 0; par < 2; ++par) {  // no capture among the timed steps
+        if ((settled ? g->sexec : g->gexec)[par]) continue;
+        const int rc = group_capture(g, par, !settled);
         if (rc) return rc;
       }
       GROUP_TRY(g, cudaEventRecord(g->t0, g->stream));
       for (int k = 0; k < 2; ++k) {
-        const int rc = group_step(g);
+        const int rc = step();
         if (rc) return rc;
       }
       GROUP_TRY(g, cudaEventRecord(g->t1, g->stream));
@@ -2325,14 +2410,13 @@ int lbmpsm_group_run_fixed(lbmpsm_group* g, int nsteps) {
       float ms = 0.f;
       GROUP_TRY(g, cudaEventElapsedTime(&ms, g->t0, g->t1));
       g->tune_ms[plan] = ms / 2;
-      nsteps -= 4;
     }
     const int best = g->tune_ms[1] <= g->tune_ms[0] ? 1 : 0;
     if (best != g->plan_pref) group_drop(g);
     g->plan_pref = best;
   }
-  for (int s = 0; s < nsteps; ++s) {
-    const int rc = group_step(g);
+  while (nsteps > 0) {
+    const int rc = step();
     if (rc) return rc;
   }
   // the members' later work is ordered after the group's

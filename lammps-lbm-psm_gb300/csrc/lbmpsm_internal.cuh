@@ -345,6 +345,8 @@ struct MapParams {
                       // third with the image index in w), written by cell_sort
   long long list_cap;
   unsigned long long* pair_total;  // [0] cell-list pairs, [1] solid-fraction codes, [2] shell nodes
+  unsigned long long* changed;     // optional: set to 1 when the map changes a slot id (only
+                                   // asked of images held in place, where few nodes write it)
   unsigned short* sfcode;          // codes of all (image, box node) pairs
   long long sf_cap;
   const double* sf_value;          // sf_value[n] = n/10^d (n = 0..1000), FP64

@@ -644,6 +644,7 @@ __global__ void __launch_bounds__(512) node_apply_kernel(MapParams p) {
     }
   }
   if (ids_dirty) {
+    if (p.changed) *p.changed = 1;
     p.tab.ids[n] = make_int2(id[0], id[1]);
     p.tab.flag[n] = (uint8_t)((id[0] > 0 ? 1 : 0) | (id[1] > 0 ? 2 : 0));
   }
@@ -714,6 +715,7 @@ struct Apply32 {
 
   __device__ __forceinline__ void store(const MapParams& p, long long n) const {
     if (ids_dirty) {
+      if (p.changed) *p.changed = 1;
       p.tab.ids[n] = make_int2(id0, id1);
       p.tab.flag[n] = (uint8_t)((id0 > 0 ? 1 : 0) | (id1 > 0 ? 2 : 0));
     }
