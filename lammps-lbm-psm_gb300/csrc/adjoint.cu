@@ -88,33 +88,54 @@ __device__ __forceinline__ void slot_weights(double e0, double e1, bool occ0, bo
   }
 }
 
+// The lattice's directions as opposite pairs (q(k), o(k)), e_q = +1 on its
+// first axis.
+template <class L>
+struct PairOf {
+  static constexpr int N = (L::Q - 1) / 2;
+  __host__ __device__ static constexpr int q(int k) {
+    return L::Q == 19 ? 2 * k + 1 : (k == 0 ? 1 : (k == 1 ? 2 : (k == 2 ? 5 : 8)));
+  }
+  __host__ __device__ static constexpr int o(int k) { return L::opp(q(k)); }
+};
+
 // Moments of v_q = w_q mu_q: M0 = sum v, M1_a = sum v e_a,
-// M2 = sum v e_a e_b in the order xx, yy, zz, xy, xz, yz.
+// M2 = sum v e_a e_b in the order xx, yy, zz, xy, xz, yz, from the sums and
+// differences of opposite directions (the weights applied to their totals).
 template <class L>
 __device__ __forceinline__ void moments(const double* mu, double& M0, double M1[3],
                                         double M2[6]) {
-  M0 = 0.0;
+  double s0[2] = {0.0, 0.0}, s1[2][3], s2[2][6];  // [axis | diagonal directions]
 #pragma unroll
-  for (int a = 0; a < 3; ++a) M1[a] = 0.0;
+  for (int c = 0; c < 2; ++c) {
 #pragma unroll
-  for (int a = 0; a < 6; ++a) M2[a] = 0.0;
+    for (int a = 0; a < 3; ++a) s1[c][a] = 0.0;
 #pragma unroll
-  for (int q = 0; q < L::Q; ++q) {
-    constexpr int dummy = 0;
-    (void)dummy;
-    const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-    const double v = L::w(q) * mu[q];
-    M0 += v;
-    if (cx) M1[0] += cx > 0 ? v : -v;
-    if (cy) M1[1] += cy > 0 ? v : -v;
-    if (cz) M1[2] += cz > 0 ? v : -v;
-    if (cx) M2[0] += v;
-    if (cy) M2[1] += v;
-    if (cz) M2[2] += v;
-    if (cx && cy) M2[3] += cx * cy > 0 ? v : -v;
-    if (cx && cz) M2[4] += cx * cz > 0 ? v : -v;
-    if (cy && cz) M2[5] += cy * cz > 0 ? v : -v;
+    for (int a = 0; a < 6; ++a) s2[c][a] = 0.0;
   }
+#pragma unroll
+  for (int k = 0; k < PairOf<L>::N; ++k) {
+    const int q = PairOf<L>::q(k);
+    const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
+    const int c = cx * cx + cy * cy + cz * cz == 1 ? 0 : 1;
+    const double s = mu[q] + mu[PairOf<L>::o(k)], d = mu[q] - mu[PairOf<L>::o(k)];
+    s0[c] += s;
+    if (cx) s1[c][0] += cx > 0 ? d : -d;
+    if (cy) s1[c][1] += cy > 0 ? d : -d;
+    if (cz) s1[c][2] += cz > 0 ? d : -d;
+    if (cx) s2[c][0] += s;
+    if (cy) s2[c][1] += s;
+    if (cz) s2[c][2] += s;
+    if (cx && cy) s2[c][3] += cx * cy > 0 ? s : -s;
+    if (cx && cz) s2[c][4] += cx * cz > 0 ? s : -s;
+    if (cy && cz) s2[c][5] += cy * cz > 0 ? s : -s;
+  }
+  const double wa = L::w(1), wd = L::w(L::Q - 1);
+  M0 = L::w(0) * mu[0] + wa * s0[0] + wd * s0[1];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) M1[a] = wa * s1[0][a] + wd * s1[1][a];
+#pragma unroll
+  for (int a = 0; a < 6; ++a) M2[a] = a < 3 ? wa * s2[0][a] + wd * s2[1][a] : wd * s2[1][a];
 }
 
 __device__ __forceinline__ void m2_times(const double M2[6], const double a[3], double out[3]) {
@@ -129,26 +150,43 @@ __device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
 
 template <class L, int q>
 __device__ __forceinline__ double edot_c(const double v[3]) {
-  double s = 0.0;
+  // (-0 is the identity of IEEE addition: the leading term costs nothing)
+  double s = -0.0;
   if (L::ex(q)) s += L::ex(q) > 0 ? v[0] : -v[0];
   if (L::ey(q)) s += L::ey(q) > 0 ? v[1] : -v[1];
   if (L::ez(q)) s += L::ez(q) > 0 ? v[2] : -v[2];
   return s;
 }
 
-template <class L, int q>
-struct Unroll {
+template <class L, int k>
+struct UnrollPairs {
   template <class Fn>
   __device__ __forceinline__ static void run(Fn& fn) {
-    fn.template apply<q>();
-    Unroll<L, q + 1>::run(fn);
+    fn.template apply<k>();
+    UnrollPairs<L, k + 1>::run(fn);
   }
 };
 template <class L>
-struct Unroll<L, L::Q> {
+struct UnrollPairs<L, PairOf<L>::N> {
   template <class Fn>
   __device__ __forceinline__ static void run(Fn&) {}
 };
+
+// rho = sum f and m = sum f e, from the sums and differences of opposite directions
+template <class L>
+__device__ __forceinline__ void density_momentum(const double* f, double& rho, double m[3]) {
+  rho = f[0];
+  m[0] = m[1] = m[2] = -0.0;
+#pragma unroll
+  for (int k = 0; k < PairOf<L>::N; ++k) {
+    const int q = PairOf<L>::q(k);
+    const double d = f[q] - f[PairOf<L>::o(k)];
+    rho += f[q] + f[PairOf<L>::o(k)];
+    if (L::ex(q)) m[0] += L::ex(q) > 0 ? d : -d;
+    if (L::ey(q)) m[1] += L::ey(q) > 0 ? d : -d;
+    if (L::ez(q)) m[2] += L::ez(q) > 0 ? d : -d;
+  }
+}
 
 // the pre-collision populations of node n in A-A storage, as the FP64
 // collide kernel reads them
@@ -219,19 +257,40 @@ __device__ __forceinline__ void node_slots(const AdjParams& p, long long n, Node
   }
 }
 
-// deterministic block sum of ADJ_PART values into this block's slot
-__device__ __forceinline__ void block_accumulate(double (&v)[ADJ_PART], double* part) {
+// deterministic block sum of the first N of ADJ_PART values into this block's
+// slot: within a warp the first levels halve the values each lane carries
+// (9 FP64 additions for five values, 5 for one)
+template <int N>
+__device__ __forceinline__ void block_accumulate(const double (&v)[ADJ_PART], double* part) {
   __shared__ double red[ADJ_THREADS / 32][ADJ_PART];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (N == 1) {
+    double x = v[0];
 #pragma unroll
-  for (int k = 0; k < ADJ_PART; ++k) {
-    double x = v[k];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) red[wid][0] = x;
+  } else {
+    static_assert(ADJ_PART <= 8, "values");
+    double w[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[wid][k] = x;
+    for (int k = 0; k < 8; ++k) w[k] = k < ADJ_PART ? v[k < ADJ_PART ? k : 0] : 0.0;
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1) {  // lane bits 16, 8, 4 choose value bits 4, 2, 1
+      const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+      for (int k = 0; k < h; ++k) {
+        const double keep = up ? w[k + h] : w[k], send = up ? w[k] : w[k + h];
+        w[k] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+      }
+    }
+    double x = w[0];
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    const int k = lane >> 2;
+    if ((lane & 3) == 0 && k < ADJ_PART) red[wid][k] = x;
   }
   __syncthreads();
-  if (threadIdx.x < ADJ_PART) {
+  if (threadIdx.x < N) {
     double x = 0.0;
 #pragma unroll
     for (int w = 0; w < ADJ_THREADS / 32; ++w) x += red[w][threadIdx.x];
@@ -240,36 +299,33 @@ __device__ __forceinline__ void block_accumulate(double (&v)[ADJ_PART], double* 
 }
 
 // ------------------------------------------------------------ reverse step
+// out_q = (1 - omega) mu_q + base + e_q.V, e.V once per pair of directions
 template <class L>
-struct AdjQ {
-  // inputs
+struct AdjPairs {
   const double* mu;
-  double omBt, omw, inv_rho, uAu;
-  double Aj[3], Au[3], cB[2], dus[2];
-  double base;  // (1-w) mu term is per q; base = A_rho + sum_s B_s A_s - uAu/rho + drag const
-  double coef;  // drag coefficient of d.e_q
-  const double* d;
+  double omw, base;
+  const double* V;
   double* out;
-  template <int q>
+  template <int k>
   __device__ __forceinline__ void apply() {
-    const double ej = edot_c<L, q>(Aj);
-    const double eAu = edot_c<L, q>(Au);
-    const double de = edot_c<L, q>(d);
-    out[q] = omw * mu[q] + omBt * ej + base + eAu * inv_rho + coef * de;
+    constexpr int q = PairOf<L>::q(k), o = PairOf<L>::o(k);
+    const double eV = edot_c<L, q>(V);
+    out[q] = omw * mu[q] + base + eV;
+    out[o] = omw * mu[o] + base - eV;
   }
 };
 
+// Bound by the FP64 pipe, as the collide: moments from the sums and
+// differences of opposite directions, the per-direction terms gathered into
+// one vector, nodes dealt out to blocks without regard to rows (56^3: 117 us a
+// step; every direction on its own and rows of 56 nodes to a block: 197 us).
 template <class L>
 __global__ void __launch_bounds__(ADJ_THREADS) adj_step_kernel(AdjParams p) {
   constexpr int Q = L::Q;
   const Geom& g = p.g;
-  const int xblocks = (g.S[0] + ADJ_THREADS - 1) / ADJ_THREADS;
-  const int row = blockIdx.x / xblocks;
-  const int sx = (blockIdx.x - row * xblocks) * ADJ_THREADS + threadIdx.x;
+  int sx, sy, sz;
   double acc[ADJ_PART] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (sx < g.S[0]) {
-    const int sy = row % g.S[1];
-    const int sz = row / g.S[1];
+  if (node_of_block<ADJ_THREADS>(g, blockIdx.x, sx, sy, sz)) {
     const long long n = node_index(g, sx, sy, sz);
     const Nbr nb = make_nbr(g, sx, sy, sz);
     const long long Np = g.Np;
@@ -281,15 +337,10 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_step_kernel(AdjParams p) {
 #pragma unroll
     for (int q = 0; q < Q; ++q)
       mu[q] = p.lin[q * Np + n + nbr_off(nb, L::ex(q), L::ey(q), L::ez(q))];
-    double rho = 0.0, m[3] = {0.0, 0.0, 0.0}, smf = 0.0;
+    double rho, m[3], smf = mu[0] * f[0];
+    density_momentum<L>(f, rho, m);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      rho += f[q];
-      smf += mu[q] * f[q];
-      if (L::ex(q)) m[0] += L::ex(q) > 0 ? f[q] : -f[q];
-      if (L::ey(q)) m[1] += L::ey(q) > 0 ? f[q] : -f[q];
-      if (L::ez(q)) m[2] += L::ez(q) > 0 ? f[q] : -f[q];
-    }
+    for (int q = 1; q < Q; ++q) smf += mu[q] * f[q];
     const double inv_rho = 1.0 / rho;
     double u[3];
 #pragma unroll
@@ -340,22 +391,18 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_step_kernel(AdjParams p) {
       p.an.sigma[2 * n] += beta[0];
       p.an.sigma[2 * n + 1] += beta[1];
     }
-    AdjQ<L> fn;
+    double V[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) V[a] = (omega - Bt) * Aj[a] + Au[a] * inv_rho + coef * d[a];
+    AdjPairs<L> fn;
     fn.mu = mu;
     fn.omw = 1.0 - omega;
-    fn.omBt = omega - Bt;
-    fn.inv_rho = inv_rho;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      fn.Aj[a] = Aj[a];
-      fn.Au[a] = Au[a];
-    }
     fn.base = (omega - Bt) * A_rho + sumBAs - dot3(u, Au) * inv_rho + dconst;
-    fn.coef = coef;
-    fn.d = d;
+    fn.V = V;
     double out[Q];
     fn.out = out;
-    Unroll<L, 0>::run(fn);
+    out[0] = fn.omw * mu[0] + fn.base;
+    UnrollPairs<L, 0>::run(fn);
 #pragma unroll
     for (int q = 0; q < Q; ++q) p.lout[q * Np + n] = out[q];
 
@@ -366,21 +413,42 @@ __global__ void __launch_bounds__(ADJ_THREADS) adj_step_kernel(AdjParams p) {
       acc[2 + a] = (omega - Bt) * Aj[a] * 0.5 + gp * Aj[a] + Au[a] * (0.5 * inv_rho) +
                    sum_cB * (1.0 - omega) * d[a] * 0.5;
   }
-  block_accumulate(acc, p.part);
+  block_accumulate<ADJ_PART>(acc, p.part);
 }
 
 // ------------------------------------------------------------ tangent step
+// The tangent of direction q, dC_q, has a part even in e and one odd in e:
+//   even: w [K + (e.u)(e.W1) + (e.F)(e.W2) + sum_k (e.us_k)(e.Y_k)]
+//   odd : w e.V
+// with K, V, W1, W2, Y_k sums over the node, so that a pair of opposite
+// directions shares everything but the last addition (48^3: 96 us a step; every
+// direction on its own and rows of 48 nodes to a block: 326 us).
+template <class L>
+struct TanPairs {
+  const double *u, *F, *V, *W1, *W2, (*us)[3], (*Y)[3];
+  double K, omw, domega;
+  bool slots;
+  const double *f, *fd;
+  double* out;
+  template <int k>
+  __device__ __forceinline__ void apply() {
+    constexpr int q = PairOf<L>::q(k), o = PairOf<L>::o(k);
+    double even = K + edot_c<L, q>(u) * edot_c<L, q>(W1) + edot_c<L, q>(F) * edot_c<L, q>(W2);
+    if (slots)
+      even += edot_c<L, q>(us[0]) * edot_c<L, q>(Y[0]) + edot_c<L, q>(us[1]) * edot_c<L, q>(Y[1]);
+    const double odd = edot_c<L, q>(V), w = L::w(q);
+    out[q] = omw * fd[q] - domega * f[q] + w * (even + odd);
+    out[o] = omw * fd[o] - domega * f[o] + w * (even - odd);
+  }
+};
+
 template <class L>
 __global__ void __launch_bounds__(ADJ_THREADS) tan_step_kernel(AdjParams p) {
   constexpr int Q = L::Q;
   const Geom& g = p.g;
-  const int xblocks = (g.S[0] + ADJ_THREADS - 1) / ADJ_THREADS;
-  const int row = blockIdx.x / xblocks;
-  const int sx = (blockIdx.x - row * xblocks) * ADJ_THREADS + threadIdx.x;
+  int sx, sy, sz;
   double acc[ADJ_PART] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (sx < g.S[0]) {
-    const int sy = row % g.S[1];
-    const int sz = row / g.S[1];
+  if (node_of_block<ADJ_THREADS>(g, blockIdx.x, sx, sy, sz)) {
     const long long n = node_index(g, sx, sy, sz);
     const Nbr nb = make_nbr(g, sx, sy, sz);
     const long long Np = g.Np;
@@ -392,15 +460,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) tan_step_kernel(AdjParams p) {
     load_state<L>(p.state, Np, n, nb, p.odd, f);
 #pragma unroll
     for (int q = 0; q < Q; ++q) fd[q] = p.lin[q * Np + n];
-    double rho = 0.0, rhod = 0.0, m[3] = {0.0, 0.0, 0.0}, md[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      rho += f[q];
-      rhod += fd[q];
-      if (L::ex(q)) { m[0] += L::ex(q) > 0 ? f[q] : -f[q]; md[0] += L::ex(q) > 0 ? fd[q] : -fd[q]; }
-      if (L::ey(q)) { m[1] += L::ey(q) > 0 ? f[q] : -f[q]; md[1] += L::ey(q) > 0 ? fd[q] : -fd[q]; }
-      if (L::ez(q)) { m[2] += L::ez(q) > 0 ? f[q] : -f[q]; md[2] += L::ez(q) > 0 ? fd[q] : -fd[q]; }
-    }
+    double rho, rhod, m[3], md[3];
+    density_momentum<L>(f, rho, m);
+    density_momentum<L>(fd, rhod, md);
     const double inv_rho = 1.0 / rho;
     double u[3], jd[3], ud[3];
 #pragma unroll
@@ -424,34 +486,49 @@ __global__ void __launch_bounds__(ADJ_THREADS) tan_step_kernel(AdjParams p) {
     }
     const double Bt = sl.B[0] + sl.B[1], Btd = Bd[0] + Bd[1];
     const double gp = 1.0 - 0.5 * omega;
-    const double hs[2] = {1.5 * dot3(sl.us[0], sl.us[0]), 1.5 * dot3(sl.us[1], sl.us[1])};
     const double rr = rhod * inv_rho;
-    double out[Q];
+    const double cf = domega - Btd, ob = omega - Bt;  // factors of feq and of its tangent
+    TanPairs<L> fn;
+    fn.K = cf * rho * (1.0 - 1.5 * usq) + ob * (rhod * (1.0 + 1.5 * usq) - 3.0 * ujd) +
+           1.5 * domega * uF - 3.0 * gp * (Fud + udF);
+    const double a1 = 4.5 * (cf * rho - ob * rhod);
+    double V[3], W1[3], W2[3], Y[2][3];
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int cx = L::ex(q), cy = L::ey(q), cz = L::ez(q);
-      const double w = L::w(q);
-      const double eu = cx * u[0] + cy * u[1] + cz * u[2];
-      const double ejd = cx * jd[0] + cy * jd[1] + cz * jd[2];
-      const double eF = cx * F[0] + cy * F[1] + cz * F[2];
-      const double eud = cx * ud[0] + cy * ud[1] + cz * ud[2];
-      const double edF = cx * dFv[0] + cy * dFv[1] + cz * dFv[2];
-      const double feq = rho * w * (1.0 + 3.0 * eu + 4.5 * eu * eu - 1.5 * usq);
-      const double feqd = w * (rhod * (1.0 - 4.5 * eu * eu + 1.5 * usq) + 3.0 * ejd +
-                               9.0 * eu * ejd - 3.0 * ujd);
-      const double gq = w * (3.0 * (eF - uF) + 9.0 * eu * eF);
-      const double gqd = w * (-3.0 * Fud + 9.0 * eF * eud + 3.0 * (edF - udF) + 9.0 * eu * edF);
-      double c = (1.0 - omega) * fd[q] - domega * f[q] + (domega - Btd) * feq +
-                 (omega - Bt) * feqd - 0.5 * domega * gq + gp * gqd;
+    for (int a = 0; a < 3; ++a) {
+      V[a] = 3.0 * (cf * rho * u[a] + ob * jd[a] - 0.5 * domega * F[a] + gp * dFv[a]);
+      W1[a] = a1 * u[a] + 9.0 * (ob * jd[a] + gp * dFv[a]) - 4.5 * domega * F[a];
+      W2[a] = 9.0 * gp * ud[a];
+      Y[0][a] = Y[1][a] = 0.0;
+    }
+    fn.slots = sl.live[0] || sl.live[1];
+    if (fn.slots) {
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         if (!sl.live[k]) continue;
-        const double evs = cx * sl.us[k][0] + cy * sl.us[k][1] + cz * sl.us[k][2];
-        const double fs = rho * w * (1.0 + 3.0 * evs + 4.5 * evs * evs - hs[k]);
-        c += Bd[k] * fs + sl.B[k] * fs * rr;
+        const double ck = rho * (Bd[k] + sl.B[k] * rr);
+        fn.K += ck * (1.0 - 1.5 * dot3(sl.us[k], sl.us[k]));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          V[a] += 3.0 * ck * sl.us[k][a];
+          Y[k][a] = 4.5 * ck * sl.us[k][a];
+        }
       }
-      out[q] = c;
     }
+    double out[Q];
+    fn.u = u;
+    fn.F = F;
+    fn.V = V;
+    fn.W1 = W1;
+    fn.W2 = W2;
+    fn.us = sl.us;
+    fn.Y = Y;
+    fn.omw = 1.0 - omega;
+    fn.domega = domega;
+    fn.f = f;
+    fn.fd = fd;
+    fn.out = out;
+    out[0] = fn.omw * fd[0] - domega * f[0] + L::w(0) * fn.K;
+    UnrollPairs<L, 0>::run(fn);
 #pragma unroll
     for (int q = 0; q < Q; ++q)
       p.lout[q * Np + n + nbr_off(nb, L::ex(q), L::ey(q), L::ez(q))] = out[q];
@@ -470,7 +547,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) tan_step_kernel(AdjParams p) {
     }
     acc[0] = dJ;
   }
-  block_accumulate(acc, p.part);
+  block_accumulate<1>(acc, p.part);
 }
 
 // ------------------------------------------------------- entries and weights
@@ -736,7 +813,7 @@ __global__ void __launch_bounds__(SUM_THREADS) adj_sum_kernel(const double* part
 }  // namespace
 
 long long adj_blocks(const Geom& g) {
-  return (long long)((g.S[0] + ADJ_THREADS - 1) / ADJ_THREADS) * g.S[1] * g.S[2];
+  return ((long long)g.S[0] * g.S[1] * g.S[2] + ADJ_THREADS - 1) / ADJ_THREADS;
 }
 
 cudaError_t launch_adj_entries(const AdjSetup& s, cudaStream_t st) {

@@ -384,29 +384,11 @@ __device__ __forceinline__ void collide_f64_node(NodeCols<L, FORCE>& s, const Co
   }
 }
 
-// Node of thread t of block b when the stored nodes (x fastest, without the
-// rows' padding) are dealt out 128 to a block: rows shorter than a block, or
-// not a multiple of a warp, leave no lane of the FP64 pipe idle.
-__device__ __forceinline__ bool node_of(const Geom& g, unsigned b, int& sx, int& sy, int& sz) {
-  const unsigned S0 = (unsigned)g.S[0];
-  const unsigned first = b * (unsigned)F64_THREADS;  // the node count stays below 2^32 (memory)
-  unsigned row = first / S0;
-  unsigned x = first - row * S0 + threadIdx.x;
-  const unsigned up = x / S0;
-  x -= up * S0;
-  row += up;
-  const unsigned z = row / (unsigned)g.S[1];
-  sx = (int)x;
-  sy = (int)(row - z * (unsigned)g.S[1]);
-  sz = (int)z;
-  return z < (unsigned)g.S[2];
-}
-
 template <class L, bool ODD, bool FORCE>
 __global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_kernel(CollideParams p) {
   __shared__ NodeCols<L, FORCE> s;
   int sx, sy, sz;
-  if (!node_of(p.g, blockIdx.x, sx, sy, sz)) return;
+  if (!node_of_block<F64_THREADS>(p.g, blockIdx.x, sx, sy, sz)) return;
   collide_f64_node<L, ODD, FORCE>(s, p, sx, sy, sz);
 }
 
@@ -421,7 +403,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_multi_ker
   while (m + 1 < mc.nm && b >= mc.first[m + 1]) ++m;
   const CollideParams& p = mc.m[m].p;
   int sx, sy, sz;
-  if (!node_of(p.g, (unsigned)(b - mc.first[m]), sx, sy, sz)) return;
+  if (!node_of_block<F64_THREADS>(p.g, (unsigned)(b - mc.first[m]), sx, sy, sz)) return;
   collide_f64_node<L, ODD, FORCE>(s, p, sx, sy, sz);
 }
 

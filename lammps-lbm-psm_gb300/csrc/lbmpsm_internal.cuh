@@ -175,6 +175,25 @@ __device__ __forceinline__ bool nbr_ok(const Nbr& nb, int cx, int cy, int cz) {
   return ok;
 }
 
+// Node of a thread of block b when the stored nodes (x fastest, without the
+// rows' padding) are dealt out THREADS to a block: rows shorter than a block, or
+// not a multiple of a warp, leave no lane idle.
+template <int THREADS>
+__device__ __forceinline__ bool node_of_block(const Geom& g, unsigned b, int& sx, int& sy, int& sz) {
+  const unsigned S0 = (unsigned)g.S[0];
+  const unsigned first = b * (unsigned)THREADS;  // the node count stays below 2^32 (memory)
+  unsigned row = first / S0;
+  unsigned x = first - row * S0 + threadIdx.x;
+  const unsigned up = x / S0;
+  x -= up * S0;
+  row += up;
+  const unsigned z = row / (unsigned)g.S[1];
+  sx = (int)x;
+  sy = (int)(row - z * (unsigned)g.S[1]);
+  sz = (int)z;
+  return z < (unsigned)g.S[2];
+}
+
 // ---------------------------------------------------------------- particle table
 struct Table {
   uint8_t* flag;   // N
