@@ -24,7 +24,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=o
           os.path.join(ROOT, "include")]
 # units whose FP64 arithmetic must not be contracted into FMAs
 NO_FMA = {"collide_f64", "particles", "layout"}
-UNITS = ["collide_f64", "collide_lowp", "particles", "layout", "adjoint", "capi"]
+UNITS = ["collide_f64", "collide_f32", "collide_f16", "collide_bf16", "collide_lowp", "particles", "layout", "adjoint", "capi"]
 
 
 def nvcc() -> str:
@@ -36,6 +36,7 @@ def nvcc() -> str:
 
 def _deps(unit: str) -> list[str]:
     return [os.path.join(CSRC, unit + ".cu"), os.path.join(CSRC, "lbmpsm_internal.cuh"),
+            os.path.join(CSRC, "collide_lowp.cuh"),
             os.path.join(CSRC, "solid_fraction.cuh"),
             os.path.join(CSRC, "fixed_f64.cuh"),
             os.path.join(ROOT, "include", "lbmpsm.h")]

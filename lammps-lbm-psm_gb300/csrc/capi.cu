@@ -481,6 +481,7 @@ int maybe_tune(lbmpsm_handle* h) {
   CUDA_TRY(h, cudaStreamIsCapturing(h->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone) return LBMPSM_OK;
   h->tune_pending = false;
+  if (tune_candidates(h->g, h->opt.storage, h->sm_count) < 2) return LBMPSM_OK;  // no choice
   void* scratch = nullptr;
   const size_t bytes = storage_bytes(h->opt.storage) * (size_t)h->g.Np * h->g.Q;
   if (cudaMalloc(&scratch, bytes) != cudaSuccess) {

@@ -226,7 +226,9 @@ struct BoxParams {
 struct PipeConfig {
   int grid = 0, threads = 0, stages = 0;
   size_t smem = 0;
-  int dy = 0, dz = 0;  // grid = dz * S1 + dy
+  int k = 1, tpp = 0;  // x-rows per tile, tiles per plane
+  FastDiv fS0{};       // division by the row length
+  int dj = 0, dz = 0;  // grid = dz * tpp + dj
 };
 
 struct CollideParams {
@@ -475,10 +477,20 @@ cudaError_t launch_collide_bf16(const CollideParams& p, int odd, cudaStream_t st
 // the direct kernel, cfg left empty)
 cudaError_t prepare_collide_lowp(const Geom& g, int storage, int sm_count, int stages,
                                  PipeConfig* cfg);
+cudaError_t prepare_collide_f32(const Geom& g, int sm_count, int stages, PipeConfig* cfg);
+cudaError_t prepare_collide_f16(const Geom& g, int sm_count, int stages, PipeConfig* cfg);
+cudaError_t prepare_collide_bf16(const Geom& g, int sm_count, int stages, PipeConfig* cfg);
+cudaError_t prepare_multi_f32(MultiCollide& mc, MultiMember* members, int sm_count);
+cudaError_t prepare_multi_f16(MultiCollide& mc, MultiMember* members, int sm_count);
+cudaError_t prepare_multi_bf16(MultiCollide& mc, MultiMember* members, int sm_count);
+cudaError_t launch_multi_f32(const MultiCollide& mc, int odd, cudaStream_t st);
+cudaError_t launch_multi_f16(const MultiCollide& mc, int odd, cudaStream_t st);
+cudaError_t launch_multi_bf16(const MultiCollide& mc, int odd, cudaStream_t st);
 // times the candidate launch shapes (pipeline stages 3, 2, 4, 5) on p.f and
 // stores the fastest in best (unchanged if none fits), the per-pair times in
 // ms_out (-1: shape does not fit)
 constexpr int LBMPSM_TUNE_CANDIDATES = 4;
+int tune_candidates(const Geom& g, int storage, int sm_count);  // how many of them fit
 cudaError_t tune_collide_lowp(CollideParams p, int storage, int sm_count, cudaStream_t st,
                               PipeConfig* best, float* ms_out);
 // one launch over the members of mc (storage 0: FP64, 1: FP32, 2: FP16, 3: BF16);
