@@ -481,7 +481,8 @@ int maybe_tune(lbmpsm_handle* h) {
   CUDA_TRY(h, cudaStreamIsCapturing(h->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone) return LBMPSM_OK;
   h->tune_pending = false;
-  if (tune_candidates(h->g, h->opt.storage, h->sm_count) < 2) return LBMPSM_OK;  // no choice
+  PipeConfig shape[LBMPSM_TUNE_CANDIDATES];
+  if (tune_shapes(h->g, h->opt.storage, h->sm_count, shape) < 2) return LBMPSM_OK;  // no choice
   void* scratch = nullptr;
   const size_t bytes = storage_bytes(h->opt.storage) * (size_t)h->g.Np * h->g.Q;
   if (cudaMalloc(&scratch, bytes) != cudaSuccess) {
@@ -501,7 +502,7 @@ int maybe_tune(lbmpsm_handle* h) {
   p.status = h->d_status;
   PipeConfig best = h->pipe;
   cudaError_t e = cudaMemcpyAsync(scratch, h->f, bytes, cudaMemcpyDeviceToDevice, h->stream);
-  if (e == cudaSuccess) e = tune_collide_lowp(p, h->opt.storage, h->sm_count, h->stream, &best, h->tune_ms);
+  if (e == cudaSuccess) e = tune_collide_lowp(p, h->opt.storage, h->stream, shape, &best, h->tune_ms);
   cudaStreamSynchronize(h->stream);
   cudaFree(scratch);
   CUDA_TRY(h, e);

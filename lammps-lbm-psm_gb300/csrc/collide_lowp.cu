@@ -42,30 +42,31 @@ cudaError_t launch_collide_multi(const MultiCollide& mc, int storage, int odd, c
 // step pairs on p.f (a scratch copy of the populations), timed with CUDA
 // events on the stream; the fastest is kept.  The candidates are one template
 // (only the stage count and the launch bounds differ), so they round alike
-// and the choice changes speed only, never results.  The direct kernel (the
-// fallback for rows longer than one staged block) is not a candidate: it
-// inlines the same node arithmetic into another kernel, where the compiler's
-// multiply-add contraction may round differently.
+// and the choice changes speed only, never results.  The direct kernel rounds
+// |u_s|^2 in another order and is not a candidate.
+//
+// One pair untimed, then one timed, three where a pair is shorter than 200 us
+// or so (a rate of 3 TB/s assumed).
 static const int cand[LBMPSM_TUNE_CANDIDATES] = {3, 2, 4, 5};
 
-// the candidate shapes that fit a lattice (grid 0: does not), each stage count once
-static cudaError_t candidate(const Geom& g, int storage, int sm_count, int k, PipeConfig* c) {
-  const cudaError_t e = prepare_collide_lowp(g, storage, sm_count, cand[k], c);
-  if (e == cudaSuccess && c->stages != cand[k]) *c = PipeConfig{};
-  return e;
-}
-
-int tune_candidates(const Geom& g, int storage, int sm_count) {
+int tune_shapes(const Geom& g, int storage, int sm_count, PipeConfig (&shape)[LBMPSM_TUNE_CANDIDATES]) {
   int n = 0;
   for (int k = 0; k < LBMPSM_TUNE_CANDIDATES; ++k) {
-    PipeConfig c{};
-    if (candidate(g, storage, sm_count, k, &c) == cudaSuccess && c.grid > 0) ++n;
+    PipeConfig& c = shape[k];
+    // (a long row has one shape whatever the stages asked for)
+    if (prepare_collide_lowp(g, storage, sm_count, cand[k], &c) != cudaSuccess || c.stages != cand[k])
+      c = PipeConfig{};
+    if (c.grid > 0) ++n;
   }
+  cudaGetLastError();
   return n;
 }
 
-cudaError_t tune_collide_lowp(CollideParams p, int storage, int sm_count, cudaStream_t st,
-                              PipeConfig* best, float* ms_out) {
+cudaError_t tune_collide_lowp(CollideParams p, int storage, cudaStream_t st,
+                              const PipeConfig (&shape)[LBMPSM_TUNE_CANDIDATES], PipeConfig* best,
+                              float* ms_out) {
+  const double pair_bytes = 4.0 * p.g.Q * (storage == 1 ? 4 : 2) * (double)p.g.N;
+  const int reps = pair_bytes < 3e12 * 200e-6 ? 3 : 1;
   cudaEvent_t e0, e1;
   cudaError_t e = cudaEventCreate(&e0);
   if (e != cudaSuccess) return e;
@@ -77,8 +78,7 @@ cudaError_t tune_collide_lowp(CollideParams p, int storage, int sm_count, cudaSt
   bool have = false;
   for (int k = 0; k < LBMPSM_TUNE_CANDIDATES; ++k) {
     ms_out[k] = -1.0f;
-    PipeConfig c{};
-    if ((e = candidate(p.g, storage, sm_count, k, &c)) != cudaSuccess) break;
+    const PipeConfig& c = shape[k];
     if (c.grid == 0) continue;  // this shape does not fit the lattice's rows
     p.pipe = c;
     auto pair = [&]() {
@@ -90,21 +90,14 @@ cudaError_t tune_collide_lowp(CollideParams p, int storage, int sm_count, cudaSt
         else
           launch_collide_f16(p, odd, st);
     };
-    // one pair untimed, one timed; three where a pair is too short to time alone
-    float ms = 0.0f;
-    int reps = 1;
     pair();
-    for (;;) {
-      cudaEventRecord(e0, st);
-      for (int r = 0; r < reps; ++r) pair();
-      cudaEventRecord(e1, st);
-      if ((e = cudaEventSynchronize(e1)) != cudaSuccess) break;
-      if ((e = cudaGetLastError()) != cudaSuccess) break;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (reps > 1 || ms > 0.2f) break;
-      reps = 3;
-    }
-    if (e != cudaSuccess) break;
+    cudaEventRecord(e0, st);
+    for (int r = 0; r < reps; ++r) pair();
+    cudaEventRecord(e1, st);
+    if ((e = cudaEventSynchronize(e1)) != cudaSuccess) break;
+    if ((e = cudaGetLastError()) != cudaSuccess) break;
+    float ms = 0.0f;
+    cudaEventElapsedTime(&ms, e0, e1);
     ms_out[k] = ms / (float)reps;
     if (!have || ms_out[k] < best_ms) {
       best_ms = ms_out[k];

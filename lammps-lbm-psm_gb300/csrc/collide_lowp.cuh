@@ -458,7 +458,7 @@ __device__ __forceinline__ bool mbar_wait_abortable(unsigned bar, unsigned phase
 // Warp-specialised pipeline of the collide / A-A stream step.  A persistent
 // grid; every block walks its tiles t, t + G, t + 2G, ... through NST
 // shared-memory stages of Q populations per node.  A tile is
-//   ONE_ROW  : one x-row of up to 256 nodes;
+//   ONE_ROW, ONE_SHORT_ROW: one x-row of up to 256, 128 nodes;
 //   SOME_ROWS: p.pipe.k consecutive rows of a plane, as many as fit 256 nodes,
 //     so that short rows fill the block and its copies (rows of 32 nodes one at
 //     a time moved 128 bytes a copy and kept one consumer warp a block: the
@@ -482,7 +482,11 @@ __device__ __forceinline__ bool mbar_wait_abortable(unsigned bar, unsigned phase
 // (after p.full_wait_limit polls) raise a shared abort flag, which ends the
 // producer's wait for their signal at once; the producer then waits, with
 // its own long limit, only for the loads it has issued.
-enum PipeMode { ONE_ROW, SOME_ROWS, LONG_ROW };
+enum PipeMode { ONE_ROW, ONE_SHORT_ROW, SOME_ROWS, LONG_ROW };
+// Staged nodes of one direction: fixed (but for long rows), so that the
+// consumers' 38 shared-memory addresses a node are two or three registers and
+// constants.
+__host__ __device__ constexpr int pipe_stride(int mode) { return mode == LONG_ROW ? 0 : (mode == ONE_SHORT_ROW ? 128 : 256); }
 template <class L, typename T, bool ODD, bool FORCE, int NST, int MINB, int MODE>
 __global__ void __launch_bounds__(PIPE_CONSUMERS + 32, MINB) collide_pipe_kernel(CollideParams p) {
   static_assert(NST >= 2, "stages");
@@ -499,7 +503,8 @@ __global__ void __launch_bounds__(PIPE_CONSUMERS + 32, MINB) collide_pipe_kernel
   const int gdj = p.pipe.dj, gdz = p.pipe.dz;
   const int ncons = (int)blockDim.x - 32;
   const unsigned row_bytes = (unsigned)(P0 * sizeof(T));
-  const unsigned dir_bytes = (unsigned)k * row_bytes;  // one direction of a stage
+  const int SD = MODE == LONG_ROW ? P0 : pipe_stride(MODE);  // staged nodes of one direction
+  const unsigned dir_bytes = (unsigned)(SD * (int)sizeof(T));
   const unsigned stage_bytes = (unsigned)Q * dir_bytes;
   const unsigned smem0 = smem_addr(smem_raw);
   T* __restrict__ F = static_cast<T*>(p.f);
@@ -621,7 +626,6 @@ __global__ void __launch_bounds__(PIPE_CONSUMERS + 32, MINB) collide_pipe_kernel
   }
 
   // -------------------------------------------------------------- consumers
-  const int SD = k * P0;  // staged nodes of one direction
   const int row = MODE == SOME_ROWS ? (int)fast_div((unsigned)tid, p.pipe.fS0) : 0;  // of the tile
   const int x0 = tid - row * S0;
   int cj = blockIdx.x % tpp, cz = blockIdx.x / tpp;
@@ -1081,7 +1085,7 @@ static cudaError_t pipe_prepare(const Geom& g, int sm_count, int k, PipeConfig* 
   const int chunks = (g.S[0] + PIPE_CONSUMERS - 1) / PIPE_CONSUMERS;
   const int nodes = MODE == LONG_ROW ? (g.S[0] + chunks - 1) / chunks : k * g.S[0];
   const int threads = (nodes + 31) / 32 * 32 + 32;  // consumers + producer warp
-  const size_t smem = (size_t)NST * L::Q * k * g.P0 * sizeof(T);
+  const size_t smem = (size_t)NST * L::Q * (MODE == LONG_ROW ? g.P0 : pipe_stride(MODE)) * sizeof(T);
   cudaError_t e;
   const void* fns[4] = {(const void*)collide_pipe_kernel<L, T, false, false, NST, MINB, MODE>,
                         (const void*)collide_pipe_kernel<L, T, false, true, NST, MINB, MODE>,
@@ -1115,7 +1119,7 @@ static cudaError_t pipe_prepare(const Geom& g, int sm_count, int k, PipeConfig* 
 // than the fuller copies gain).
 static int tile_rows(const Geom& g, int blocks) {
   const long long nrows = (long long)g.S[1] * g.S[2];
-  int k = std::max(1, std::min(PIPE_CONSUMERS / g.S[0], g.S[1]));
+  int k = std::max(1, std::min(PIPE_CONSUMERS / g.P0, g.S[1]));  // (of the padded rows)
   while (k > 1 && nrows / k < 4ll * blocks) --k;
   return k;
 }
@@ -1136,10 +1140,17 @@ static cudaError_t with_shape(const Geom& g, int stages, int k, Fn fn) {
   typedef std::integral_constant<int, 5> I5;
   typedef std::integral_constant<int, B> IB;
   typedef std::integral_constant<int, ONE_ROW> One;
+  typedef std::integral_constant<int, ONE_SHORT_ROW> Short;
   typedef std::integral_constant<int, SOME_ROWS> Some;
   typedef std::integral_constant<int, LONG_ROW> Long;
   if (g.S[0] > PIPE_CONSUMERS) return stages == 2 ? fn(I2(), I2(), Long()) : fn(I3(), I2(), Long());
   if (k > 1) return stages == 2 ? fn(I2(), IB(), Some()) : fn(I3(), IB(), Some());
+  if (g.P0 <= pipe_stride(ONE_SHORT_ROW)) switch (stages) {
+    case 2: return fn(I2(), IB(), Short());
+    case 4: return fn(I4(), I2(), Short());
+    case 5: return fn(I5(), I2(), Short());
+    default: return fn(I3(), IB(), Short());
+  }
   switch (stages) {
     case 2: return fn(I2(), IB(), One());
     case 4: return fn(I4(), I2(), One());

@@ -490,9 +490,11 @@ cudaError_t launch_multi_bf16(const MultiCollide& mc, int odd, cudaStream_t st);
 // stores the fastest in best (unchanged if none fits), the per-pair times in
 // ms_out (-1: shape does not fit)
 constexpr int LBMPSM_TUNE_CANDIDATES = 4;
-int tune_candidates(const Geom& g, int storage, int sm_count);  // how many of them fit
-cudaError_t tune_collide_lowp(CollideParams p, int storage, int sm_count, cudaStream_t st,
-                              PipeConfig* best, float* ms_out);
+// the shapes that fit a lattice (grid 0: does not); returns how many
+int tune_shapes(const Geom& g, int storage, int sm_count, PipeConfig (&shape)[LBMPSM_TUNE_CANDIDATES]);
+cudaError_t tune_collide_lowp(CollideParams p, int storage, cudaStream_t st,
+                              const PipeConfig (&shape)[LBMPSM_TUNE_CANDIDATES], PipeConfig* best,
+                              float* ms_out);
 // one launch over the members of mc (storage 0: FP64, 1: FP32, 2: FP16, 3: BF16);
 // prepare_collide_multi fills mc.first, tcp, pipe and the members' k / tpp
 // from their geometries (host copies in members) and the device's occupancy
