@@ -222,7 +222,9 @@ void* lbmpsm_stream(lbmpsm_handle* h);
  * staged through pinned memory and copied (devices without that access, or
  * the environment variable LBMPSM_HOST_STAGING=1 at lbmpsm_create); -1 for
  * a NULL handle.  Both give the same results bit for bit.  Single-box
- * handles only: lbmpsm_step_batch always stages. */
+ * handles only: lbmpsm_step_batch always stages.  With 1, lbmpsm_get_populations,
+ * lbmpsm_set_populations and lbmpsm_export_fields also work on the caller's
+ * arrays. */
 int lbmpsm_host_direct(const lbmpsm_handle* h);
 
 /* Run nsteps coupling steps with the particle images already on the device

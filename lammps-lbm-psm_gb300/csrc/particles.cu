@@ -1267,55 +1267,58 @@ cudaError_t launch_table_export(const Geom& g, const Table& t, int* ids, double*
   return cudaGetLastError();
 }
 
-// execute_write_vti field read (src/fix_LBM_PSM_writeVTI.h:146-169)
-__global__ void export_fields_kernel(Geom g, Table t, const double* rho, const double* u,
-                                     int as_double, double B0, double rho0, double u0,
-                                     void* solid_out, void* rho_out, void* u_out) {
-  const int nxi = g.L[0] - 2, nyi = g.L[1] - 2, nzi = g.dim == 3 ? g.L[2] - 2 : 1;
-  const long long total = (long long)nxi * nyi * nzi;
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= total) return;
-  const int i = 1 + (int)(id % nxi);
-  const int j = 1 + (int)((id / nxi) % nyi);
-  const int k = (g.dim == 3 ? 1 : 0) + (int)(id / ((long long)nxi * nyi));
-  const int sx = i - g.off[0], sy = j - g.off[1], sz = k - g.off[2];
-  const long long n = node_index(g, sx, sy, sz);
-  const double2 e = t.eps ? t.eps[n] : make_double2(t.rec32[2 * n].x, t.rec32[2 * n + 1].x);
-  const double Bv = (e.x + e.y);
-  const double sv = (Bv > 1.0 ? 1.0 : Bv) * B0;
-  const double rv = (rho ? rho[n] : 1.0) * rho0;
-  const double ux = (u ? u[3 * n + 0] : 0.0) * u0;
-  const double uy = (u ? u[3 * n + 1] : 0.0) * u0;
-  const double uz = g.dim == 3 ? (u ? u[3 * n + 2] : 0.0) * u0 : 0.0;
-  if (as_double) {
-    if (solid_out) static_cast<double*>(solid_out)[id] = sv;
-    if (rho_out) static_cast<double*>(rho_out)[id] = rv;
-    if (u_out) {
-      double* uo = static_cast<double*>(u_out);
-      uo[3 * id + 0] = ux;
-      uo[3 * id + 1] = uy;
-      uo[3 * id + 2] = uz;
+// execute_write_vti field read (src/fix_LBM_PSM_writeVTI.h:146-169): z
+// outermost, x innermost.  One block per 256 nodes of an x-row; the velocities
+// (three values a node) go through shared memory, so that every field leaves in
+// full runs, to device memory or, over NVLink-C2C, to the caller's arrays.
+constexpr int EXP_THREADS = 256;
+template <typename T>
+__global__ void __launch_bounds__(EXP_THREADS) export_fields_kernel(Geom g, Table t, const double* rho,
+                                                                    const double* u, double B0, double rho0,
+                                                                    double u0, T* solid_out, T* rho_out,
+                                                                    T* u_out) {
+  __shared__ T su[3 * EXP_THREADS];
+  const int nxi = g.L[0] - 2, nyi = g.L[1] - 2;
+  const int xblocks = (nxi + EXP_THREADS - 1) / EXP_THREADS;
+  const unsigned row = blockIdx.x / (unsigned)xblocks;
+  const int x0 = (int)(blockIdx.x - row * (unsigned)xblocks) * EXP_THREADS;
+  const int k = (int)(row / (unsigned)nyi), j = (int)(row - (unsigned)k * (unsigned)nyi);
+  const int cnt = min(EXP_THREADS, nxi - x0), tid = threadIdx.x;
+  const long long id0 = (long long)row * nxi + x0;
+  if (tid < cnt) {
+    const long long n = node_index(g, 1 + x0 + tid - g.off[0], 1 + j - g.off[1],
+                                   (g.dim == 3 ? 1 : 0) + k - g.off[2]);
+    if (solid_out) {
+      const double2 e = t.eps ? t.eps[n] : make_double2(t.rec32[2 * n].x, t.rec32[2 * n + 1].x);
+      const double Bv = (e.x + e.y);
+      solid_out[id0 + tid] = (T)((Bv > 1.0 ? 1.0 : Bv) * B0);
     }
-  } else {
-    if (solid_out) static_cast<float*>(solid_out)[id] = (float)sv;
-    if (rho_out) static_cast<float*>(rho_out)[id] = (float)rv;
+    if (rho_out) rho_out[id0 + tid] = (T)((rho ? rho[n] : 1.0) * rho0);
     if (u_out) {
-      float* uo = static_cast<float*>(u_out);
-      uo[3 * id + 0] = (float)ux;
-      uo[3 * id + 1] = (float)uy;
-      uo[3 * id + 2] = g.dim == 3 ? (float)uz : 0.0f;
+      su[3 * tid] = (T)((u ? u[3 * n + 0] : 0.0) * u0);
+      su[3 * tid + 1] = (T)((u ? u[3 * n + 1] : 0.0) * u0);
+      su[3 * tid + 2] = g.dim == 3 ? (T)((u ? u[3 * n + 2] : 0.0) * u0) : (T)0;
     }
   }
+  if (!u_out) return;
+  __syncthreads();
+  for (int c = tid; c < 3 * cnt; c += EXP_THREADS) u_out[3 * id0 + c] = su[c];
 }
 
 cudaError_t launch_export_fields(const Geom& g, const Table& t, const double* rho, const double* u,
                                  int as_double, double B0, double rho0, double u0, void* solid_out,
                                  void* rho_out, void* u_out, cudaStream_t st) {
-  const long long total =
-      (long long)(g.L[0] - 2) * (g.L[1] - 2) * (g.dim == 3 ? g.L[2] - 2 : 1);
-  if (total <= 0) return cudaSuccess;
-  export_fields_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-      g, t, rho, u, as_double, B0, rho0, u0, solid_out, rho_out, u_out);
+  const long long rows = (long long)(g.L[1] - 2) * (g.dim == 3 ? g.L[2] - 2 : 1);
+  if (rows <= 0 || g.L[0] <= 2) return cudaSuccess;
+  const unsigned grid = (unsigned)(rows * ((g.L[0] - 2 + EXP_THREADS - 1) / EXP_THREADS));
+  if (as_double)
+    export_fields_kernel<double><<<grid, EXP_THREADS, 0, st>>>(
+        g, t, rho, u, B0, rho0, u0, static_cast<double*>(solid_out), static_cast<double*>(rho_out),
+        static_cast<double*>(u_out));
+  else
+    export_fields_kernel<float><<<grid, EXP_THREADS, 0, st>>>(
+        g, t, rho, u, B0, rho0, u0, static_cast<float*>(solid_out), static_cast<float*>(rho_out),
+        static_cast<float*>(u_out));
   return cudaGetLastError();
 }
 
