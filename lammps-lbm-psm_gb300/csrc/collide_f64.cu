@@ -384,11 +384,52 @@ __device__ __forceinline__ void collide_f64_node(NodeCols<L, FORCE>& s, const Co
   }
 }
 
+// Deals the nodes of block b to its threads (every thread of the block calls):
+// those of two particles first, those of one, then the fluid.  A node of a
+// sphere costs more than twice a fluid one and a warp takes the loop of its
+// dearest node; spheres cut most rows, so that with nodes in order 42% of the
+// warps took the PSM loop where 17% of the nodes needed it, dealt out 23%
+// (128 x 96 x 160 nodes, 230 spheres: 1190 -> 1000 us a step).  The accesses stay
+// within the block's cache lines, and no other node reads or writes a node's
+// slots.
+__device__ __forceinline__ bool dealt_node(const CollideParams& p, unsigned b, int& sx, int& sy,
+                                           int& sz) {
+  constexpr int W = F64_THREADS / 32;
+  __shared__ unsigned char order[F64_THREADS];
+  __shared__ int count[3][W];
+  const int t = threadIdx.x, w = t >> 5;
+  const bool in = node_of_block<F64_THREADS>(p.g, b, sx, sy, sz);
+  const unsigned flag = in ? p.tab.flag[node_index(p.g, sx, sy, sz)] : 0u;
+  if (!__syncthreads_or(flag != 0u)) return in;
+  const int cls = !in ? 3 : ((flag & 2u) ? 0 : (flag ? 1 : 2));
+  int before = 0;  // nodes of the class in the warp's lower lanes
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+    if ((t & 31) == 0) count[c][w] = __popc(m);
+    if (cls == c) before = __popc(m & ((1u << (t & 31)) - 1u));
+  }
+  __syncthreads();
+  int total = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const int m = count[c][k];
+      if (c < cls || (c == cls && k < w)) before += m;
+      total += m;
+    }
+  if (in) order[before] = (unsigned char)t;
+  __syncthreads();
+  if (t >= total) return false;
+  return node_of_block<F64_THREADS>(p.g, b, sx, sy, sz, order[t]);
+}
+
 template <class L, bool ODD, bool FORCE>
 __global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_kernel(CollideParams p) {
   __shared__ NodeCols<L, FORCE> s;
   int sx, sy, sz;
-  if (!node_of_block<F64_THREADS>(p.g, blockIdx.x, sx, sy, sz)) return;
+  if (!dealt_node(p, blockIdx.x, sx, sy, sz)) return;
   collide_f64_node<L, ODD, FORCE>(s, p, sx, sy, sz);
 }
 
@@ -403,7 +444,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_multi_ker
   while (m + 1 < mc.nm && b >= mc.first[m + 1]) ++m;
   const CollideParams& p = mc.m[m].p;
   int sx, sy, sz;
-  if (!node_of_block<F64_THREADS>(p.g, (unsigned)(b - mc.first[m]), sx, sy, sz)) return;
+  if (!dealt_node(p, (unsigned)(b - mc.first[m]), sx, sy, sz)) return;
   collide_f64_node<L, ODD, FORCE>(s, p, sx, sy, sz);
 }
 

@@ -175,15 +175,16 @@ __device__ __forceinline__ bool nbr_ok(const Nbr& nb, int cx, int cy, int cz) {
   return ok;
 }
 
-// Node of a thread of block b when the stored nodes (x fastest, without the
-// rows' padding) are dealt out THREADS to a block: rows shorter than a block, or
-// not a multiple of a warp, leave no lane idle.
+// Node k (a thread's own by default) of block b when the stored nodes (x fastest,
+// without the rows' padding) are dealt out THREADS to a block: rows shorter than
+// a block, or not a multiple of a warp, leave no lane idle.
 template <int THREADS>
-__device__ __forceinline__ bool node_of_block(const Geom& g, unsigned b, int& sx, int& sy, int& sz) {
+__device__ __forceinline__ bool node_of_block(const Geom& g, unsigned b, int& sx, int& sy, int& sz,
+                                              unsigned k) {
   const unsigned S0 = (unsigned)g.S[0];
   const unsigned first = b * (unsigned)THREADS;  // the node count stays below 2^32 (memory)
   unsigned row = first / S0;
-  unsigned x = first - row * S0 + threadIdx.x;
+  unsigned x = first - row * S0 + k;
   const unsigned up = x / S0;
   x -= up * S0;
   row += up;
@@ -192,6 +193,10 @@ __device__ __forceinline__ bool node_of_block(const Geom& g, unsigned b, int& sx
   sy = (int)(row - z * (unsigned)g.S[1]);
   sz = (int)z;
   return z < (unsigned)g.S[2];
+}
+template <int THREADS>
+__device__ __forceinline__ bool node_of_block(const Geom& g, unsigned b, int& sx, int& sy, int& sz) {
+  return node_of_block<THREADS>(g, b, sx, sy, sz, threadIdx.x);
 }
 
 // ---------------------------------------------------------------- particle table
