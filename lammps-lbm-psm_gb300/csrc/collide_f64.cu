@@ -89,9 +89,8 @@ struct NodeCols {
 
 // What the directions of one node share besides.
 struct NodeF64 {
-  double half[3];     // 0.5*|v|^2*invCs2 of the fluid and of the slots
-  fx::u64 half62[3];  // the same aligned (fixed-point factors)
-  double rw[3];       // rho*w of the rest, axis and diagonal weights
+  double vv[3];  // v.v of the fluid and of the slots
+  double rw[3];  // rho*w of the rest, axis and diagonal weights
   double B[2], oneMinusBtot;
 };
 
@@ -101,38 +100,41 @@ __device__ __forceinline__ double pair_dot(const PairDesc& d, const double (*v)[
   return d.s2 == 0 ? x : x + turned(v[d.i2][t], d.s2 < 0);
 }
 
-// The equilibria rw*(1 +- 3 e.v + 4.5 (e.v)^2 - 1.5 v.v) of a pair: e.v, its
-// multiple and its square are formed once, the opposite direction taking them
-// with the sign turned (negation is exact, so both round as when formed
-// alone; 0.5*invCs4 is exact).  FX: the sums on the integer units
-// (fixed_f64.cuh), the same bits.
-template <bool FX>
-__device__ __forceinline__ void pair_feq(double ev, double invCs2, double h4, double half,
-                                         fx::u64 half62, double rw, double& plus, double& minus) {
-  const double a = ev * invCs2, b = ev * ev * h4;
-  if (FX) {
-    fx::factors(a, b, half62, plus, minus);
-  } else {
-    plus = (1.0 + a) + b - half;
-    minus = (1.0 - a) + b - half;
-  }
-  plus = rw * plus;
-  minus = rw * minus;
+// The equilibria rw*(1 +- 3 e.v + 4.5 (e.v)^2 - 1.5 v.v) of a pair minus its
+// populations: e.v, its multiple and its square are formed once, the opposite
+// direction taking them with the sign turned (negation is exact, so both round
+// as when formed alone; 0.5*invCs4 is exact).
+__device__ __forceinline__ void pair_diff(double ev, const CollideParams& p, double half, double rw,
+                                          double fp, double fm, double& dp, double& dm) {
+  const double a = ev * p.invCs2, b = ev * ev * (0.5 * p.invCs4);
+  dp = rw * ((1.0 + a) + b - half) - fp;
+  dm = rw * ((1.0 - a) + b - half) - fm;
+}
+
+// The same on the integer units (fixed_f64.cuh), but for one product: the
+// constants are 3 and 4.5 exactly.
+static_assert(1.0 / (1.0 / 3.0) == 3.0 && 1.0 / ((1.0 / 3.0) * (1.0 / 3.0)) == 9.0, "");
+__device__ __forceinline__ void pair_diff62(double ev, fx::u64 half, fx::u64 rw, fx::u64 fp, fx::u64 fm,
+                                            double& dp, double& dm) {
+  fx::u64 plus, minus;
+  fx::factors(ev, ev * ev, half, plus, minus);
+  dp = fx::difference62(fx::product62(rw, plus), fp);
+  dm = fx::difference62(fx::product62(rw, minus), fm);
 }
 
 // fi after collision (collisionAndStream, src/LBM_PSM_BGK_dynamics.h:40-114)
-// with NS slots (0: plain BGK); t: B*Omega_s per slot.
+// with NS slots (0: plain BGK); d and ds: feq - fi of the fluid and of the slot
+// velocities; t: B*Omega_s per slot.
 template <int NS>
-__device__ __forceinline__ double relaxed(double fi, double feq, const double (&f0s)[2],
+__device__ __forceinline__ double relaxed(double fi, double d, const double (&ds)[2],
                                           const NodeF64& nd, double omega, double omo,
                                           double (&t)[2]) {
-  const double d = feq - fi;
   if (NS == 0) return fi + d * omega;
   const double od = omo * d;  // one_minus_omega*(fi - feq) is -od bit for bit
   double r = fi + nd.oneMinusBtot * d * omega;
 #pragma unroll
   for (int n = 0; n < NS; ++n) {
-    t[n] = nd.B[n] * ((f0s[n] - fi) - od);
+    t[n] = nd.B[n] * (ds[n] - od);
     r = r + t[n];
   }
   return r;
@@ -145,34 +147,63 @@ __device__ __forceinline__ void collide_dirs(NodeCols<L, FORCE>& s, int t, const
                                              const CollideParams& p, const BoxParams& bp,
                                              bool has_force) {
   const double pref = bp.guo_pref, omega = bp.omega, omo = bp.one_minus_omega;
-  const double invCs2 = p.invCs2, invCs4 = p.invCs4, h4 = 0.5 * p.invCs4;
+  const double invCs2 = p.invCs2, invCs4 = p.invCs4;
+  double half[1 + NS];  // 0.5*v.v*invCs2 of the fluid and of the slots
+  fx::u64 half62[1 + NS], rw62[3];
+#pragma unroll
+  for (int n = 0; n <= NS; ++n) {
+    if (FX)
+      half62[n] = fx::times62<3, 1>(nd.vv[n]);
+    else
+      half[n] = 0.5 * nd.vv[n] * invCs2;
+  }
+  if (FX) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) rw62[c] = fx::to64(nd.rw[c]);
+  }
   auto guo = [&](int g0, int g1, int g2, double w, double last) {
     const double a = s.g[g0][t] + s.g[3 + g1][t] + s.g[6 + g2][t];
     return pref * (w * (a * invCs2 + last));
   };
   {  // the rest population
-    double f0s[2] = {0.0, 0.0}, bo[2];
-    const double feq = nd.rw[0] * (FX ? fx::one_minus(nd.half62[0]) : 1.0 - nd.half[0]);
+    const double fi = s.f[0][t];
+    double d[1 + NS], ds[2] = {0.0, 0.0}, bo[2];
 #pragma unroll
-    for (int n = 0; n < NS; ++n)
-      f0s[n] = nd.rw[0] * (FX ? fx::one_minus(nd.half62[1 + n]) : 1.0 - nd.half[1 + n]);
-    double r = relaxed<NS>(s.f[0][t], feq, f0s, nd, omega, omo, bo);
+    for (int n = 0; n <= NS; ++n)
+      d[n] = FX ? fx::difference62(fx::product62(rw62[0], fx::one_minus(half62[n])), fx::to62(fi))
+                : nd.rw[0] * (1.0 - half[n]) - fi;
+#pragma unroll
+    for (int n = 0; n < NS; ++n) ds[n] = d[1 + n];
+    double r = relaxed<NS>(fi, d[0], ds, nd, omega, omo, bo);
     if (FORCE) r = r + guo(0, 0, 0, L::w(0), 0.0);
     s.f[0][t] = r;
   }
 #pragma unroll 1
   for (int k = 0; k < (L::Q - 1) / 2; ++k) {
     const PairDesc& d = pair_desc<L>(k);
-    const double rw = d.s2 == 0 ? nd.rw[1] : nd.rw[2];
     const double eu = pair_dot(d, s.u, t);
-    double ep, em, sp[2] = {0.0, 0.0}, sm[2] = {0.0, 0.0}, tp[2], tm[2];
-    pair_feq<FX>(eu, invCs2, h4, nd.half[0], nd.half62[0], rw, ep, em);
+    const double fi = s.f[d.q][t], fo = s.f[d.o][t];
+    double dp[1 + NS], dm[1 + NS], sp[2] = {0.0, 0.0}, sm[2] = {0.0, 0.0}, tp[2], tm[2];
+    if (FX) {
+      const fx::u64 fi62 = fx::to62(fi), fo62 = fx::to62(fo), rw = d.s2 == 0 ? rw62[1] : rw62[2];
 #pragma unroll
-    for (int n = 0; n < NS; ++n)  // feq(iq, rho, uSolid) (src/LBM_PSM_dynamics.h:72-85)
-      pair_feq<FX>(pair_dot(d, s.us[n], t), invCs2, h4, nd.half[1 + n], nd.half62[1 + n], rw, sp[n],
-                   sm[n]);
-    double fp = relaxed<NS>(s.f[d.q][t], ep, sp, nd, omega, omo, tp);
-    double fm = relaxed<NS>(s.f[d.o][t], em, sm, nd, omega, omo, tm);
+      for (int n = 0; n <= NS; ++n)  // feq(iq, rho, uSolid) (src/LBM_PSM_dynamics.h:72-85)
+        pair_diff62(n == 0 ? eu : pair_dot(d, s.us[n > 0 ? n - 1 : 0], t), half62[n], rw, fi62, fo62,
+                    dp[n], dm[n]);
+    } else {
+      const double rw = d.s2 == 0 ? nd.rw[1] : nd.rw[2];
+#pragma unroll
+      for (int n = 0; n <= NS; ++n)
+        pair_diff(n == 0 ? eu : pair_dot(d, s.us[n > 0 ? n - 1 : 0], t), p, half[n], rw, fi, fo, dp[n],
+                  dm[n]);
+    }
+#pragma unroll
+    for (int n = 0; n < NS; ++n) {
+      sp[n] = dp[1 + n];
+      sm[n] = dm[1 + n];
+    }
+    double fp = relaxed<NS>(fi, dp[0], sp, nd, omega, omo, tp);
+    double fm = relaxed<NS>(fo, dm[0], sm, nd, omega, omo, tm);
     if (FORCE) {
       const double w = d.s2 == 0 ? L::w(1) : L::w(L::Q - 1);
       const double eF = has_force ? bp.eF[(L::Q == 9 ? 9 : 0) + k] : 0.0;
@@ -287,8 +318,7 @@ __device__ __forceinline__ void collide_f64_node(NodeCols<L, FORCE>& s, const Co
     for (int c = 0; c < 3; ++c) p.u_out[3 * n + c] = u[c];
   }
   NodeF64 nd;
-  nd.half[0] = 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]) * p.invCs2;
-  nd.half62[0] = fx::align62(nd.half[0]);
+  nd.vv[0] = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     near = near && fx::slow(u[c]);
@@ -349,8 +379,7 @@ __device__ __forceinline__ void collide_f64_node(NodeCols<L, FORCE>& s, const Co
         }
         near = near && fx::slow(v[c]);
       }
-      nd.half[1 + k] = 0.5 * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * p.invCs2;
-      nd.half62[1 + k] = fx::align62(nd.half[1 + k]);
+      nd.vv[1 + k] = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
     }
     const bool one = !__any_sync(act, (flag & 2) != 0);
     if (__all_sync(act, near)) {

@@ -1,14 +1,16 @@
-// fixed_f64.cuh -- IEEE double additions of the collide step on the integer
-// units, bit for bit.
+// fixed_f64.cuh -- IEEE double additions and some products of the collide step on
+// the integer units, bit for bit.
 //
 // This GPU issues 1.68 FP64 operations per clock and multiprocessor against
 // about 100 integer ones, and both at once, so an addition whose rounding
 // position is known can be had for a dozen integer instructions beside the
 // FP64 pipe.  Near rest it is known: populations, their sums and the factors
 // 1 + 3 e.u + ... of the equilibria keep to a few binades.  The values are held
-// as 64-bit integers in units of 2^-61 (populations and sums) or 2^-62 (the
-// factors); each result is rounded to 53 significant bits, ties to even, as
-// the IEEE addition it stands for.  Every function states the range it needs;
+// as 64-bit integers in units of 2^-61 (density and momentum sums) or 2^-62 (the
+// factors, equilibria and their differences from the populations); each result
+// is rounded to 53 significant bits, ties to even, as the IEEE operation it
+// stands for.  Products by the constants 3, 4.5 and 1.5 and of a density with a
+// factor are formed the same way.  Every function states the range it needs;
 // the caller checks the ranges (populations in [2^-7, 1), densities above 0.9
 // and below 2, velocity components below 5/64) and takes the FP64 expressions
 // otherwise.  A suspension whose spheres move at 0.04 stays inside.
@@ -117,13 +119,23 @@ LBMPSM_HD double from61_near1(u64 t) {
   return of_bits((t >> (8 + c)) + ((u64)(1021u + c) << 52));
 }
 
-// |x| in units of 2^-62, |x| < 1/2: bits below the unit are kept as a set
-// lowest bit ("sticky"), which rounds like them at any position above bit 1
-LBMPSM_HD u64 align62(double x) {
+// |x * K / 2^H| rounded as a double, in units of 2^-62 (K/2^H = 3, 4.5 or 1.5;
+// |x| <= 5/32): the 53 bits of the product are formed with the significand's
+// multiple; bits below the unit are kept as a set lowest bit ("sticky"), which
+// rounds like them at any position above bit 1.  (A product in the denormal
+// range is all sticky.)
+template <int K, int H>
+LBMPSM_HD u64 times62(double x) {
+  static_assert(K == 3 || K == 9, "");
   const u64 b = bits_of(x);
   const unsigned e = (unsigned)(b >> 52) & 0x7FFu;
-  const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull)) << 8;
-  const unsigned r0 = 1021u - e;
+  u64 m = (b & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull);
+  m = K == 3 ? m + (m << 1) : m + (m << 3);  // the leading bit at 53 or 54 (K = 9: 55 or 56)
+  const unsigned c = (unsigned)(m >> (K == 3 ? 54 : 56)) & 1u;
+  const int sh = (K == 3 ? 1 : 3) + (int)c;
+  const u64 half = (K == 3 ? 1ull : 4ull) << c;
+  m = ((m + (half - 1ull) + ((m >> sh) & 1ull)) & ~(2ull * half - 1ull)) << 7;
+  const unsigned r0 = 1020u + H - e;
   const unsigned r = r0 < 63u ? r0 : 63u;
   const u64 a = m >> r;
   return (a << r) != m ? (a | 1ull) : a;
@@ -139,29 +151,61 @@ LBMPSM_HD u64 rne53_62(u64 s) {
   return (s + (half - 1ull) + ((s >> sh) & 1ull)) & ~(2ull * half - 1ull);
 }
 
-// the double s * 2^-62 for a 53-bit s in [1/2, 2)
-LBMPSM_HD double from62(u64 s) {
-  const unsigned c = (unsigned)(s >> 62);
-  return of_bits((s >> (9 + c)) + ((u64)(1021u + c) << 52));
-}
-
-// ((1 + a) + b) - u and ((1 - a) + b) - u, each addition rounded, for a = 3 x,
-// b = 4.5 x^2 with |x| <= 5/32 and 0 <= u < 1/24 (u aligned already): the first
-// stays in [1 - u, 3/2 + u], the second in [3/5 - u, 1]
-LBMPSM_HD void factors(double a, double b, u64 u62, double& plus, double& minus) {
-  const u64 A = align62(a), B = align62(b);
+// ((1 + 3 e) + 4.5 ee) - u and ((1 - 3 e) + 4.5 ee) - u in units of 2^-62, each
+// operation rounded, for |e| <= 5/32, ee = e*e rounded and 0 <= u < 1/24 (u
+// aligned already): the first stays in [1 - u, 3/2 + u], the second in
+// [3/5 - u, 1] (e >= 0; the other way round below)
+LBMPSM_HD void factors(double e, double ee, u64 u62, u64& plus, u64& minus) {
+  const u64 A = times62<3, 0>(e), B = times62<9, 1>(ee);
   u64 p = rne(ONE62 + A, 10);          // in [1, 3/2): units of 2^-52
   u64 m = rne(ONE62 - A, 9);           // in (1/2, 1]: units of 2^-53
   p = rne53_62(rne(p + B, 10) - u62);  // (in [1, 2) before the subtraction)
   m = rne53_62(rne53_62(m + B) - u62);
-  const double fp = from62(p), fm = from62(m);
-  const bool neg = (i64)bits_of(a) < 0;
-  plus = neg ? fm : fp;
-  minus = neg ? fp : fm;
+  const bool neg = (i64)bits_of(e) < 0;
+  plus = neg ? m : p;
+  minus = neg ? p : m;
 }
 
-// 1 - u, rounded (u aligned, below 1/24)
-LBMPSM_HD double one_minus(u64 u62) { return from62(rne(ONE62 - u62, 9)); }
+// 1 - u, rounded (u aligned, below 1/24), in units of 2^-62
+LBMPSM_HD u64 one_minus(u64 u62) { return rne(ONE62 - u62, 9); }
+
+// x in [2^-7, 1) in units of 2^-64 and of 2^-62
+LBMPSM_HD u64 to64(double x) {
+  const u64 b = bits_of(x);
+  return (((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11) >> ((1022u - (unsigned)(b >> 52)) & 63u);
+}
+LBMPSM_HD u64 to62(double x) {
+  const u64 b = bits_of(x);
+  return ((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << (((unsigned)(b >> 52) - 1013u) & 63u);
+}
+
+// the product of r (units of 2^-64) and s (units of 2^-62), rounded to 53 bits,
+// in units of 2^-62: from 2^-7 to 2, so that at least three bits of the unit
+// lie below the last place
+LBMPSM_HD u64 product62(u64 r, u64 s) {
+  const unsigned __int128 x = (unsigned __int128)r * s;
+  const u64 t = (u64)(x >> 64) | ((u64)x != 0 ? 1ull : 0ull);
+  const int sh = 11 - clz32((unsigned)(t >> 32));
+  const u64 m = (1ull << sh) - 1ull;
+  return (t + (m >> 1) + ((t >> sh) & 1ull)) & ~m;
+}
+
+// a - b rounded, as a double (units of 2^-62, both multiples of 8 below 2^63).
+// Multiples of 8 below 2^56 in size need no rounding.
+LBMPSM_HD double difference62(u64 a, u64 b) {
+  i64 t = (i64)(a - b);
+  if (abs_hi(t) >> 24) {
+    const int sh = 11 - clz32(abs_hi(t));
+    const u64 m = (1ull << sh) - 1ull;
+    t = (i64)(((u64)t + (m >> 1) + (((u64)t >> sh) & 1ull)) & ~m);
+  }
+  const u64 sg = (u64)t & 0x8000000000000000ull;
+  const u64 v = t < 0 ? (u64)0 - (u64)t : (u64)t;
+  const unsigned hi = (unsigned)(v >> 32);
+  const int lz = clz32(hi ? hi : ((unsigned)v | 1u)) + (hi ? 0 : 32);
+  const u64 d = sg | (((v << lz) >> 11) + ((u64)(1023 - lz) << 52));
+  return v == 0 ? 0.0 : of_bits(d);
+}
 
 // Density and momentum sums of compute_macro_values
 // (src/LBM_PSM_BGK_dynamics.cpp:48-77), each addition rounded in its place:

@@ -67,26 +67,41 @@ static void sums(const char* name, long n) {
 }
 
 static void factors(long n) {
-  long bad = 0;
+  long bad = 0, done = 0;
   for (long it = 0; it < n; ++it) {
     const double mag = it % 7 == 0 ? 0.0 : std::exp2(-uni(0, 70)), lim = 0.078125;
     double u[3] = {uni(-lim, lim) * (it % 3 ? 1 : mag), uni(-lim, lim) * (it % 5 ? 1 : mag), uni(-lim, lim) * mag};
     if (it % 11 == 0) u[0] = std::ldexp((double)((int)(gen() % 129) - 64), -11 - (int)(gen() % 40));
     if (it % 101 == 0) u[0] = std::ldexp(u[0], -1000 - (int)(gen() % 60));
     if (!fx::slow(u[0]) || !fx::slow(u[1])) continue;
-    const double eu = it % 2 ? u[0] + u[1] : u[0], a = eu * 3.0, b = eu * eu * 4.5;
-    const double uu = 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]) * 3.0;
+    const double eu = it % 2 ? u[0] + u[1] : u[0], a = eu * 3.0, ee = eu * eu, b = ee * 4.5;
+    const double vv = u[0] * u[0] + u[1] * u[1] + u[2] * u[2], uu = 0.5 * vv * 3.0;
     volatile double p = 1.0 + a, m = 1.0 - a, o = 1.0 - uu;
     p = p + b;
     p = p - uu;
     m = m + b;
     m = m - uu;
-    double P, M;
-    const fx::u64 u62 = fx::align62(uu);
-    fx::factors(a, b, u62, P, M);
-    if (P != p || M != m || fx::one_minus(u62) != o) ++bad;
+    // the equilibria and their differences from populations
+    const double w[4] = {1.0 / 3, 1.0 / 18, 1.0 / 36, 4.0 / 9};
+    const double rho = it % 13 == 0 ? 1.0 : uni(0.62, 1.9), rw = rho * w[it % 4];
+    volatile double fe[3] = {rw * p, rw * m, rw * o};
+    double fi = it % 3 ? fe[it % 3] * (1 + uni(-1, 1) * std::exp2(-uni(1, 50))) : uni(0.0079, 0.99);
+    if (it % 23 == 0) fi = fe[it % 3];
+    if (!(fi >= 0x1p-7 && fi < 1.0)) continue;
+    ++done;
+    volatile double d[3] = {fe[0] - fi, fe[1] - fi, fe[2] - fi};
+    fx::u64 P, M;
+    const fx::u64 u62 = fx::times62<3, 1>(vv), r64 = fx::to64(rw), f62 = fx::to62(fi), zero = 0;
+    fx::factors(eu, ee, u62, P, M);
+    const fx::u64 F[3] = {P, M, fx::one_minus(u62)};
+    if (fx::difference62(P, zero) != p || fx::difference62(M, zero) != m || fx::difference62(F[2], zero) != o) ++bad;
+    for (int k = 0; k < 3; ++k) {
+      const fx::u64 e = fx::product62(r64, F[k]);
+      if (fx::difference62(e, zero) != fe[k] || fx::difference62(e, f62) != d[k]) ++bad;
+      if (std::signbit(fx::difference62(e, f62)) != std::signbit(d[k])) ++bad;
+    }
   }
-  std::printf("factors in_range 1.000 different %ld\n", bad);
+  std::printf("factors in_range %.3f different %ld\n", (double)done / n, bad);
 }
 
 int main() {
