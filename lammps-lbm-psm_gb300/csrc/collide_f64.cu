@@ -14,7 +14,10 @@
 
 namespace lbmpsm {
 
-constexpr int F64_THREADS = 128, F64_BLOCKS = 5;  // (five blocks of columns fit the shared memory)
+constexpr int F64_THREADS = 128;
+// Blocks per multiprocessor: of the columns without a body force five (four 2%
+// slower, six spill and gain 0.6% at most), with one four (five 1% slower).
+constexpr int f64_blocks(bool force) { return force ? 4 : 5; }
 
 // Opposite directions in pairs (q, o = opp(q)), q the one whose first non-zero
 // component is +1: e_q = +1 on axis i1, s2 on axis i2 (axis pairs: s2 = 0, i2 = i1).
@@ -108,22 +111,24 @@ __device__ __forceinline__ double pair_dot(const PairDesc& d, const double (*v)[
 // populations: e.v, its multiple and its square are formed once, the opposite
 // direction taking them with the sign turned (negation is exact, so both round
 // as when formed alone; 0.5*invCs4 is exact).
-__device__ __forceinline__ void pair_diff(double ev, const CollideParams& p, double half, double rw,
-                                          double fp, double fm, double& dp, double& dm) {
+__device__ __forceinline__ double2 pair_diff(double ev, const CollideParams& p, double half, double rw,
+                                             double fp, double fm) {
   const double a = ev * p.invCs2, b = ev * ev * (0.5 * p.invCs4);
-  dp = rw * ((1.0 + a) + b - half) - fp;
-  dm = rw * ((1.0 - a) + b - half) - fm;
+  return make_double2(rw * ((1.0 + a) + b - half) - fp, rw * ((1.0 - a) + b - half) - fm);
 }
 
 // The same on the integer units (fixed_f64.cuh), but for one product: the
-// constants are 3 and 4.5 exactly.
+// constants are 3 and 4.5 exactly.  One copy of the code, called by the fluid's
+// and the slots' loops: inlined, warps of the different loops on one
+// multiprocessor waited for instruction fetches (128 x 96 x 160 nodes with 230
+// spheres: 920 us a step, called 845).
 static_assert(1.0 / (1.0 / 3.0) == 3.0 && 1.0 / ((1.0 / 3.0) * (1.0 / 3.0)) == 9.0, "");
-__device__ __forceinline__ void pair_diff62(double ev, fx::u64 half, fx::u64 rw, fx::u64 fp, fx::u64 fm,
-                                            double& dp, double& dm) {
+__device__ __noinline__ double2 pair_diff62(double ev, fx::u64 half, fx::u64 rw, fx::u64 fp,
+                                            fx::u64 fm) {
   fx::u64 plus, minus;
   fx::factors(ev, ev * ev, half, plus, minus);
-  dp = fx::difference62(fx::product62(rw, plus), fp);
-  dm = fx::difference62(fx::product62(rw, minus), fm);
+  return make_double2(fx::difference62(fx::product62(rw, plus), fp),
+                      fx::difference62(fx::product62(rw, minus), fm));
 }
 
 // fi after collision (collisionAndStream, src/LBM_PSM_BGK_dynamics.h:40-114)
@@ -215,27 +220,26 @@ __device__ __forceinline__ void collide_dirs(NodeCols<L, FORCE>& s, int t, const
     const PairDesc& d = pair_desc<L>(k);
     const double eu = pair_dot(d, s.u, t);
     const double fi = s.f[d.q][t], fo = s.f[d.o][t];
-    double dp[1 + NS], dm[1 + NS], sp[2] = {0.0, 0.0}, sm[2] = {0.0, 0.0}, tp[2], tm[2];
+    double2 dd[1 + NS];  // feq - f of both directions, the fluid's and the slots' velocities
+    double sp[2] = {0.0, 0.0}, sm[2] = {0.0, 0.0}, tp[2], tm[2];
     if (FX) {
       const fx::u64 fi62 = fx::to62(fi), fo62 = fx::to62(fo), rw = d.s2 == 0 ? rw62[1] : rw62[2];
 #pragma unroll
       for (int n = 0; n <= NS; ++n)  // feq(iq, rho, uSolid) (src/LBM_PSM_dynamics.h:72-85)
-        pair_diff62(n == 0 ? eu : pair_dot(d, s.us[n > 0 ? n - 1 : 0], t), half62[n], rw, fi62, fo62,
-                    dp[n], dm[n]);
+        dd[n] = pair_diff62(n == 0 ? eu : pair_dot(d, s.us[n > 0 ? n - 1 : 0], t), half62[n], rw, fi62, fo62);
     } else {
       const double rw = d.s2 == 0 ? nd.rw[1] : nd.rw[2];
 #pragma unroll
       for (int n = 0; n <= NS; ++n)
-        pair_diff(n == 0 ? eu : pair_dot(d, s.us[n > 0 ? n - 1 : 0], t), p, half[n], rw, fi, fo, dp[n],
-                  dm[n]);
+        dd[n] = pair_diff(n == 0 ? eu : pair_dot(d, s.us[n > 0 ? n - 1 : 0], t), p, half[n], rw, fi, fo);
     }
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
-      sp[n] = dp[1 + n];
-      sm[n] = dm[1 + n];
+      sp[n] = dd[1 + n].x;
+      sm[n] = dd[1 + n].y;
     }
-    double fp = relaxed<NS>(fi, dp[0], sp, nd, omega, omo, tp);
-    double fm = relaxed<NS>(fo, dm[0], sm, nd, omega, omo, tm);
+    double fp = relaxed<NS>(fi, dd[0].x, sp, nd, omega, omo, tp);
+    double fm = relaxed<NS>(fo, dd[0].y, sm, nd, omega, omo, tm);
     if (FORCE) {
       const int c = single ? d.g[nd.axis] : -1;
       if (c == 0) {
@@ -498,7 +502,7 @@ __device__ __forceinline__ bool dealt_node(const CollideParams& p, unsigned b, i
 }
 
 template <class L, bool ODD, bool FORCE>
-__global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_kernel(CollideParams p) {
+__global__ void __launch_bounds__(F64_THREADS, f64_blocks(FORCE)) collide_f64_kernel(CollideParams p) {
   __shared__ NodeCols<L, FORCE> s;
   int sx, sy, sz;
   if (!dealt_node(p, blockIdx.x, sx, sy, sz)) return;
@@ -509,7 +513,7 @@ __global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_kernel(Co
 // [first[m], first[m+1]), laid out as its own kernel's; every node runs the
 // same code as above, so the results are the members'.
 template <class L, bool ODD, bool FORCE>
-__global__ void __launch_bounds__(F64_THREADS, F64_BLOCKS) collide_f64_multi_kernel(MultiCollide mc) {
+__global__ void __launch_bounds__(F64_THREADS, f64_blocks(FORCE)) collide_f64_multi_kernel(MultiCollide mc) {
   __shared__ NodeCols<L, FORCE> s;
   const int b = blockIdx.x;
   int m = 0;
