@@ -1762,7 +1762,9 @@ extern "C" int lbmpsm_export_fields_static(lbmpsm_handle* h, int as_double, doub
 // The adjoint keeps the state before every checkpoint_every-th step in HBM
 // during the forward pass; the reverse pass recomputes each segment's states
 // from its checkpoint (out-of-place FP64 collides into a segment store) and
-// walks the segment backwards.  The tangent runs beside the forward pass.
+// walks the segment backwards.  The last segment's states are kept as the
+// forward pass makes them (a copy costs a tenth of a collide), and the segment
+// that is not full is the first.  The tangent runs beside the forward pass.
 namespace {
 
 struct AdjScratch {
@@ -1964,12 +1966,16 @@ int lbmpsm_adjoint_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   for (auto& l : lam) CUDA_TRY(h, sc.get(&l, state));
   CUDA_TRY(h, cudaMemsetAsync(lam[0], 0, state, h->stream));
 
-  // forward pass: the ordinary steps, a checkpoint before every K-th
+  // segment seg holds the steps first(seg) to first(seg + 1) - 1
+  auto first = [&](int seg) { return seg == 0 ? 1 : T - (nseg - seg) * K + 1; };
+  // forward pass: the ordinary steps, a checkpoint before each segment's first
   const long long ts = h->t;
   bool settled = false;
-  for (int t = 1; t <= T; ++t) {
-    if ((t - 1) % K == 0)
-      CUDA_TRY(h, cudaMemcpyAsync(ckpt[(size_t)((t - 1) / K)], h->f, state,
+  for (int t = 1, seg = 0; t <= T; ++t) {
+    if (seg < nseg && t == first(seg))
+      CUDA_TRY(h, cudaMemcpyAsync(ckpt[(size_t)seg++], h->f, state, cudaMemcpyDeviceToDevice, h->stream));
+    else if (seg == nseg)
+      CUDA_TRY(h, cudaMemcpyAsync(store[(size_t)(t - first(nseg - 1) - 1)], h->f, state,
                                   cudaMemcpyDeviceToDevice, h->stream));
     rc = enqueue_step(h, n, false, !settled, true);
     if (rc) return rc;
@@ -1993,9 +1999,9 @@ int lbmpsm_adjoint_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   AdjParams p = adj_params(h, an, part, direction);
   int cur = 0;  // lam[cur] holds lambda of the step after the one being reversed
   for (int seg = nseg - 1; seg >= 0; --seg) {
-    const int a = seg * K + 1, b = std::min(a + K - 1, T);
+    const int a = first(seg), b = first(seg + 1) - 1;
     auto st_of = [&](int t) { return t == a ? ckpt[(size_t)seg] : store[(size_t)(t - a - 1)]; };
-    for (int t = a + 1; t <= b; ++t) {
+    for (int t = a + 1; t <= b && seg < nseg - 1; ++t) {
       rc = collide_into(h, st_of(t - 1), st_of(t), (int)((ts + t - 2) & 1));
       if (rc) return rc;
     }
