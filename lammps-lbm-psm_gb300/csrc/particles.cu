@@ -90,27 +90,41 @@ __global__ void img_prep_kernel(MapParams p) {
   Img im;
   if (mine) {
     const Geom& g = p.g;
-    im.tag = p.tag[i];
+    // every input first, all in flight at once: the arrays may lie in host
+    // memory, and behind a store or a division each load waits for the one
+    // before it
+    im.bidx = p.img_box ? p.img_box[i] : 0;
+    const int tag = p.tag[i];
+    const double radius = p.radius[i];
+    double x[3], v[3], om[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      x[c] = p.x[3 * (size_t)i + c];
+      v[c] = p.v[3 * (size_t)i + c];
+      om[c] = p.omega[3 * (size_t)i + c];
+    }
+    const BoxParams& bp = p.box[im.bidx];
+    const double origin[3] = {bp.origin[0], bp.origin[1], bp.origin[2]};
+    const double Uc = bp.Uc, u_lb = bp.u_lb, tc = bp.tc, dt_d = bp.dt_d;
+    im.tag = tag;
     if (p.copy_tag) {  // the caller's arrays, kept for later steps with these images
       const size_t nn = (size_t)p.n;
-      p.copy_tag[i] = im.tag;
+      p.copy_tag[i] = tag;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        p.copy_xvw[3 * (size_t)i + c] = p.x[3 * (size_t)i + c];
-        p.copy_xvw[3 * nn + 3 * (size_t)i + c] = p.v[3 * (size_t)i + c];
-        p.copy_xvw[6 * nn + 3 * (size_t)i + c] = p.omega[3 * (size_t)i + c];
+        p.copy_xvw[3 * (size_t)i + c] = x[c];
+        p.copy_xvw[3 * nn + 3 * (size_t)i + c] = v[c];
+        p.copy_xvw[6 * nn + 3 * (size_t)i + c] = om[c];
       }
-      p.copy_xvw[9 * nn + i] = p.radius[i];
+      p.copy_xvw[9 * nn + i] = radius;
     }
-    im.bidx = p.img_box ? p.img_box[i] : 0;
     im.zoff = im.bidx * g.bz;
-    const BoxParams& bp = p.box[im.bidx];
-    const double r = p.radius[i] / p.dx;
+    const double r = radius / p.dx;
     im.r = r;
     bool valid = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const double xl = local_centre(p.x[3 * i + d], bp.origin[d], p.dx);
+      const double xl = local_centre(x[d], origin[d], p.dx);
       im.xl[d] = xl;
       int lo = (int)(xl - r) - 2;
       int hi = (int)(xl + r) + 2;
@@ -133,8 +147,8 @@ __global__ void img_prep_kernel(MapParams p) {
       im.lo[d] = slo + z0;
       im.hi[d] = shi + z0;
       if (slo >= shi) valid = false;
-      im.uT[d] = p.v[3 * i + d] / bp.Uc * bp.u_lb;
-      im.om[d] = p.omega[3 * i + d] * bp.tc * bp.dt_d;
+      im.uT[d] = v[d] / Uc * u_lb;
+      im.om[d] = om[d] * tc * dt_d;
       im.uTf[d] = (float)im.uT[d];
       im.omf[d] = (float)im.om[d];
     }
