@@ -988,8 +988,8 @@ struct Sums<true> {
 // A solo image's tag can only sit on nodes within rP (eps > 0 from this
 // image), so each row is cut to the x-range that may lie within rP: an FP32
 // bound widened by 0.01 node, a superset (extra nodes fail the tag test).  The
-// rows of the box are taken in groups of 64, one warp a group, 32 rows at a
-// time, one per lane: the warp walks the nodes of their segments 32 at a time
+// rows of the box are taken in groups (red_group), one warp a group, up to 32
+// rows at a time, one per lane: the warp walks the nodes of their segments 32 at a time
 // (x fastest, consecutive lanes on consecutive nodes), a lane finding its
 // node's row by a binary search of the segments' offsets across the warp.  The
 // lanes' sums of a group are combined in a fixed tree, the groups' sums in
@@ -1001,9 +1001,17 @@ struct Sums<true> {
 // wave); with few, eight blocks spread an image's groups over eight
 // multiprocessors, their sums meeting in the first block's shared memory (one
 // image of diameter 16: 45 us by one block).
+//
+// Rows per group: a node's FP64 sums are 27 operations on a pipe that a
+// multiprocessor's warps share, and a disc has few rows, so FP64 images take
+// small groups that reach all eight blocks (groups of 64 and 32/8: a step with
+// one disc of diameter 40 79.4 and 77.4 us, 16 tangent steps with four spheres
+// of diameter 12 3.85 and 3.71 ms); FP32 sums keep 64 (a 2-D step the same with 8).
 constexpr int RED_THREADS = 64;
-constexpr int RED_GROUP = 64;       // rows per group
-constexpr int RED_MAX_GROUPS = 32;  // groups whose sums are held at a time
+static __device__ __forceinline__ int red_group(const Geom& g, bool f64) {
+  return !f64 ? 64 : (g.dim == 2 ? 8 : 32);
+}
+constexpr int RED_MAX_GROUPS = 64;  // groups whose sums are held at a time
 constexpr int RED_CLUSTER = 8;
 
 template <bool F64, int C>
@@ -1023,7 +1031,7 @@ static __device__ __forceinline__ void reduce_image(const ReduceParams& p) {
   const int wx = bx.qhi[0] - bx.qlo[0], wy = bx.qhi[1] - bx.qlo[1], wz = bx.qhi[2] - bx.qlo[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int R = wx > 0 && wy > 0 && wz > 0 ? wy * wz : 0;  // x-rows of the box
-  const int G = (R + RED_GROUP - 1) / RED_GROUP;
+  const int group = red_group(g, F64), G = (R + group - 1) / group;
   const FastDiv fy = make_fastdiv((unsigned)max(wy, 1));
   const int xi[3] = {bx.xi[0], bx.xi[1], bx.xi[2]};  // xl = xi + xf exactly
   const float xf[3] = {bx.xf[0], bx.xf[1], bx.xf[2]};
@@ -1032,16 +1040,17 @@ static __device__ __forceinline__ void reduce_image(const ReduceParams& p) {
   Pair total = S::zero();  // thread k < 12 of the first block: sum k
   for (int g0 = 0; g0 < G || g0 == 0; g0 += RED_MAX_GROUPS) {
     const int gend = min(G, g0 + RED_MAX_GROUPS);
-    for (int gi = g0 + rank * NW + warp; gi < gend; gi += C * NW) {
+    for (int gi = g0 + warp * C + rank; gi < gend; gi += C * NW) {
+      const int rend = min(R, (gi + 1) * group);
       S acc;
       acc.clear();
 #pragma unroll 1
-      for (int r0 = gi * RED_GROUP; r0 < min(R, (gi + 1) * RED_GROUP); r0 += 32) {
+      for (int r0 = gi * group; r0 < rend; r0 += 32) {
         const int r = r0 + lane;
         int xa = bx.qlo[0], len = 0, j = 0, k = 0;
         float fdy = 0.0f, fdz = 0.0f;
         double ddy = 0.0, ddz = 0.0;
-        if (r < R) {
+        if (r < rend) {
           const int q = (int)fast_div((unsigned)r, fy);
           j = bx.qlo[1] + r - q * wy;
           k = bx.qlo[2] + q;
