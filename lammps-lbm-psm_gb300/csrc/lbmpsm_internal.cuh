@@ -381,7 +381,7 @@ struct MapParams {
   long long shell_cap;
   int sm_count;                    // multiprocessors (persistent grids)
   int* status;
-  int write32;        // also write the FP32 mirror
+  int write32;        // the table holds FP32 records (else the FP64 ones)
 };
 
 struct ReduceParams {

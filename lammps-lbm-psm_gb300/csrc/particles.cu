@@ -369,16 +369,15 @@ __global__ void cell_sort_kernel(MapParams p, int ncells) {
     }
     a[j + 1] = v;
   }
-  // the images' table-update records in list order (FP32 / FP16 storage)
-  if (p.write32)
-    for (int k = 0; k < m; ++k) {
-      const int ii = a[k];
-      int4* r = p.lrec + 3 * ((long long)off + k);
-      r[0] = p.arec[3 * ii];
-      r[1] = p.arec[3 * ii + 1];
-      const int4 u = p.arec[3 * ii + 2];
-      r[2] = make_int4(u.x, u.y, u.z, ii);
-    }
+  // the images' table-update records in list order
+  for (int k = 0; k < m; ++k) {
+    const int ii = a[k];
+    int4* r = p.lrec + 3 * ((long long)off + k);
+    r[0] = p.arec[3 * ii];
+    r[1] = p.arec[3 * ii + 1];
+    const int4 u = p.arec[3 * ii + 2];
+    r[2] = make_int4(u.x, u.y, u.z, ii);
+  }
 }
 
 // A shell node (between the early-out radii) whose sub-cells all lie on one
@@ -548,142 +547,19 @@ __global__ void __launch_bounds__(SFS_THREADS, 8) sf_shell_kernel(MapParams p) {
 // sf_old > 1e-5 means the tag matched), so only the sf bit decides.  sf > 1e-5
 // exactly when the code is non-zero.  The table is written back only where it
 // changed.
-// Bit equality of two doubles as two 32-bit compares (64-bit integer
-// compares take the slow path on this GPU).
-static __device__ __forceinline__ bool same_bits(double a, double b) {
-  return __double2loint(a) == __double2loint(b) && __double2hiint(a) == __double2hiint(b);
-}
-
-// FP64 storage: the table in FP64 (ids, eps, us) with the FP32 mirror.
-__global__ void __launch_bounds__(512) node_apply_kernel(MapParams p) {
-  const int c = (blockIdx.z * p.C[1] + blockIdx.y) * p.C[0] + blockIdx.x;
-  const int cnt = p.cell_count[c];
-  if (cnt == 0) return;
-  if (p.pair_total[0] > (unsigned long long)p.list_cap ||
-      p.pair_total[1] > (unsigned long long)p.sf_cap)
-    return;
-  const Geom& g = p.g;
-  const int sx = blockIdx.x * p.cb[0] + threadIdx.x;
-  const int sy = blockIdx.y * p.cb[1] + threadIdx.y;
-  const int sz = blockIdx.z * p.cb[2] + threadIdx.z;
-  if (sx >= g.S[0] || sy >= g.S[1] || sz >= g.S[2]) return;
-  const long long n = node_index(g, sx, sy, sz);
-  const int hi = sx + g.off[0], hj = sy + g.off[1];
-  const int hk = sz - box_of_z(g, sz) * g.bz + g.off[2];  // z in the box's own frame
-  const int* lst = p.list + p.cell_off[c];
-  int id[2] = {0, 0};
-  double eps[2] = {0.0, 0.0};
-  bool have_ids = false, have_eps = false, ids_dirty = false;
-  bool slot_dirty[2] = {false, false};
-  double us[6];
-  for (int t = 0; t < cnt; ++t) {
-    const Img& im = p.img[lst[t]];
-    if (sx < im.lo[0] || sx >= im.hi[0] || sy < im.lo[1] || sy >= im.hi[1] || sz < im.lo[2] ||
-        sz >= im.hi[2])
-      continue;
-    const int li = ((sz - im.lo[2]) * im.box[1] + (sy - im.lo[1])) * im.box[0] + (sx - im.lo[0]);
-    const unsigned short cd = p.sfcode[im.sf_off + li];
-    const int tag = im.tag;
-    if (!have_ids) {
-      const int2 v = p.tab.ids[n];
-      id[0] = v.x;
-      id[1] = v.y;
-      have_ids = true;
-    }
-    const int match = tag == id[0] ? 0 : (tag == id[1] ? 1 : -1);
-    if (cd == 0) {  // setToZero (src/LBM_PSM_lattice.cpp:302-324)
-      if (match >= 0) {
-        if (!have_eps) {
-          const double2 e = p.tab.eps[n];
-          eps[0] = e.x;
-          eps[1] = e.y;
-          have_eps = true;
-        }
-        id[match] = 0;
-        eps[match] = 0.0;
-        us[3 * match] = us[3 * match + 1] = us[3 * match + 2] = 0.0;
-        ids_dirty = true;
-        slot_dirty[match] = true;
-      }
-      continue;
-    }
-    // setParticleOnLattice: matching slot, else the first empty one, else drop
-    int slot = -1;
-    if (id[0] == tag)
-      slot = 0;
-    else if (id[1] == tag)
-      slot = 1;
-    else if (id[0] == 0)
-      slot = 0;
-    else if (id[1] == 0)
-      slot = 1;
-    if (slot < 0) continue;
-    if (!have_eps) {
-      const double2 e = p.tab.eps[n];
-      eps[0] = e.x;
-      eps[1] = e.y;
-      have_eps = true;
-    }
-    const double sf = cd == SF_ONE ? 1.0 : p.sf_value[cd];
-    // rigid-body velocity of the node (src/LBM_PSM_exchangeParticleData.cpp:83-89)
-    double u0, u1, u2;
-    if (im.has_spin) {
-      const double dx = (double)hi - im.xl[0];
-      const double dy = (double)hj - im.xl[1];
-      const double dz = (double)hk - im.xl[2];
-      u0 = im.uT[0] + im.om[1] * dz - im.om[2] * dy;
-      u1 = im.uT[1] + im.om[2] * dx - im.om[0] * dz;
-      u2 = im.uT[2] + im.om[0] * dy - im.om[1] * dx;
-    } else {
-      // every omega component +0.0 and no uT component -0.0: the reference's
-      // (uT + 0*dz) - 0*dy is uT bit for bit
-      u0 = im.uT[0];
-      u1 = im.uT[1];
-      u2 = im.uT[2];
-    }
-    // re-setting a slot to the values it already holds changes nothing
-    bool same = !slot_dirty[slot] && id[slot] == tag && same_bits(eps[slot], sf);
-    if (same) {
-      const double* cur = p.tab.us + 6 * n + 3 * slot;
-      same = same_bits(cur[0], u0) && same_bits(cur[1], u1) && same_bits(cur[2], u2);
-    }
-    if (!same) {
-      if (id[slot] != tag) ids_dirty = true;
-      id[slot] = tag;
-      eps[slot] = sf;
-      us[3 * slot + 0] = u0;
-      us[3 * slot + 1] = u1;
-      us[3 * slot + 2] = u2;
-      slot_dirty[slot] = true;
-    }
-  }
-  if (ids_dirty) {
-    if (p.changed) *p.changed = 1;
-    p.tab.ids[n] = make_int2(id[0], id[1]);
-    p.tab.flag[n] = (uint8_t)((id[0] > 0 ? 1 : 0) | (id[1] > 0 ? 2 : 0));
-  }
-  if (slot_dirty[0] || slot_dirty[1]) p.tab.eps[n] = make_double2(eps[0], eps[1]);
-  for (int b = 0; b < 2; ++b) {
-    if (!slot_dirty[b]) continue;
-    for (int k = 0; k < 3; ++k) p.tab.us[6 * n + 3 * b + k] = us[3 * b + k];
-    if (p.write32)
-      p.tab.rec32[2 * n + b] = make_float4((float)eps[b], (float)us[3 * b], (float)us[3 * b + 1],
-                                           (float)us[3 * b + 2]);
-  }
-}
-
-
-// FP32 / FP16 storage: the table is ids + the FP32 records the collide
-// kernel reads (eps, u_s per slot); the same update rules, no FP64.  The
-// records hold the FP32 roundings of the reference's values (for spinning
-// images the node velocity is formed in FP32).
+//
+// FP64 storage: the table is ids, eps and us, the reference's values bit for
+// bit.  FP32 / FP16 storage: ids and the FP32 records the collide kernel reads
+// (eps, u_s per slot), their FP32 roundings (for spinning images the node
+// velocity is formed in FP32), no FP64.
 //
 // One node's update state: the tags of its two slots as they stand after
 // the images applied so far.  Slot records are written through (the table
 // ends with the same records as when only changed ones are written, without
 // a read before the write), so only the ids live in registers; the ids and
 // the flag are written back at the end if they changed.
-struct Apply32 {
+template <bool F64>
+struct Apply {
   int id0, id1;
   bool ids_dirty;
 
@@ -693,17 +569,16 @@ struct Apply32 {
     ids_dirty = false;
   }
 
-  // one image with code cd at node n; nv.yzw is the node velocity it sets
-  __device__ __forceinline__ void image(const MapParams& p, long long n, int tag,
-                                        unsigned short cd, float4 nv) {
-    if (cd == 0) {  // setToZero (src/LBM_PSM_lattice.cpp:302-324)
+  // the slot that an image with code cd writes at this node (-1: none); cd = 0:
+  // setToZero, the slot left empty (src/LBM_PSM_lattice.cpp:302-324)
+  __device__ __forceinline__ int slot_of(int tag, unsigned short cd) {
+    if (cd == 0) {
       const int m = tag == id0 ? 0 : (tag == id1 ? 1 : -1);
       if (m >= 0) {
         if (m == 0) id0 = 0; else id1 = 0;
         ids_dirty = true;
-        p.tab.rec32[2 * n + m] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      return;
+      return m;
     }
     // setParticleOnLattice: matching slot, else the first empty one, else drop
     int slot = -1;
@@ -715,16 +590,48 @@ struct Apply32 {
       slot = 0;
     else if (id1 == 0)
       slot = 1;
-    if (slot < 0) return;
-    nv.x = cd == SF_ONE ? 1.0f : p.sf_value32[cd];
-    const int cur = slot == 0 ? id0 : id1;
-    if (cur != tag) {
+    if (slot >= 0 && (slot == 0 ? id0 : id1) != tag) {
       if (slot == 0) id0 = tag; else id1 = tag;
       ids_dirty = true;
     }
+    return slot;
+  }
+
+  // FP32: one image with code cd at node n; nv.yzw is the node velocity it sets
+  __device__ __forceinline__ void image(const MapParams& p, long long n, int tag,
+                                        unsigned short cd, float4 nv) {
+    const int slot = slot_of(tag, cd);
+    if (slot < 0) return;
+    nv.x = cd == SF_ONE ? 1.0f : p.sf_value32[cd];
     // written whether or not it changes: a store does not wait, whereas
     // reading the record first to skip an unchanged one would
-    p.tab.rec32[2 * n + slot] = nv;
+    p.tab.rec32[2 * n + slot] = cd == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : nv;
+  }
+
+  // FP64: the same at the node (hi, hj, hk) of the box's own frame
+  __device__ __forceinline__ void image(const MapParams& p, long long n, int tag, unsigned short cd,
+                                        const Img& im, bool spin, int hi, int hj, int hk) {
+    const int slot = slot_of(tag, cd);
+    if (slot < 0) return;
+    double sf = 0.0, u[3] = {0.0, 0.0, 0.0};
+    if (cd != 0) {
+      sf = cd == SF_ONE ? 1.0 : p.sf_value[cd];
+      // rigid-body velocity of the node (src/LBM_PSM_exchangeParticleData.cpp:83-89)
+      if (spin) {
+        const double dx = small_int_to_double(hi) - im.xl[0];
+        const double dy = small_int_to_double(hj) - im.xl[1];
+        const double dz = small_int_to_double(hk) - im.xl[2];
+        u[0] = im.uT[0] + im.om[1] * dz - im.om[2] * dy;
+        u[1] = im.uT[1] + im.om[2] * dx - im.om[0] * dz;
+        u[2] = im.uT[2] + im.om[0] * dy - im.om[1] * dx;
+      } else {
+        // every omega component +0.0 and no uT component -0.0: the reference's
+        // (uT + 0*dz) - 0*dy is uT bit for bit
+        for (int k = 0; k < 3; ++k) u[k] = im.uT[k];
+      }
+    }
+    reinterpret_cast<double*>(p.tab.eps)[2 * n + slot] = sf;
+    for (int k = 0; k < 3; ++k) p.tab.us[6 * n + 3 * slot + k] = u[k];
   }
 
   __device__ __forceinline__ void store(const MapParams& p, long long n) const {
@@ -755,8 +662,13 @@ static __device__ __forceinline__ float4 spin_velocity(const Img& im, int hi, in
 // fields of Img), each record serving all the thread's nodes, whose code
 // and slot record loads are independent.  The slot ids are loaded with the
 // cell's count and offset, so that they add no round of dependent loads.
-template <int NPT>
-__global__ void __launch_bounds__(512 / NPT, 8) node_apply32_kernel(MapParams p) {
+//
+// FP64 storage takes the same kernel at four blocks per multiprocessor (the
+// velocities need the registers); an image's record is read only where a node
+// is set (128 x 96 x 160 nodes, 230 spheres: 12 us a step faster than one node a
+// thread walking the images' full records).
+template <bool F64, int NPT>
+__global__ void __launch_bounds__(512 / NPT, F64 ? 4 : 8) node_apply_kernel(MapParams p) {
   const int c = (blockIdx.z * p.C[1] + blockIdx.y) * p.C[0] + blockIdx.x;
   const Geom& g = p.g;
   const int sx = blockIdx.x * p.cb[0] + threadIdx.x;
@@ -782,7 +694,7 @@ __global__ void __launch_bounds__(512 / NPT, 8) node_apply32_kernel(MapParams p)
   if (cnt == 0 || !inside) return;
   if (tot0 > (unsigned long long)p.list_cap || tot1 > (unsigned long long)p.sf_cap) return;
   const int4* __restrict__ lrec = p.lrec + 3 * (long long)coff;
-  Apply32 st[NPT];
+  Apply<F64> st[NPT];
 #pragma unroll
   for (int k = 0; k < NPT; ++k) st[k].init(ids0[k]);
   bool touched[NPT];
@@ -817,16 +729,19 @@ __global__ void __launch_bounds__(512 / NPT, 8) node_apply32_kernel(MapParams p)
       cd[k] = in[k] ? __ldg(p.sfcode + off + (sz0 + k * dz - lo2) * plane) : (unsigned short)0;
 #pragma unroll
     for (int k = 0; k < NPT; ++k) touched[k] = touched[k] || in[k];
-    if (B.w) {
+    if (F64 || B.w) {
       const int hi = sx + g.off[0], hj = sy + g.off[1];
 #pragma unroll
       for (int k = 0; k < NPT; ++k) {
         if (!in[k]) continue;
         const int z = sz0 + k * dz;
         const int hk = z - box_of_z(g, z) * g.bz + g.off[2];  // z in the box's own frame
-        st[k].image(p, n0 + k * zstride, A.w, cd[k], spin_velocity(p.img[U.w], hi, hj, hk));
+        if constexpr (F64)
+          st[k].image(p, n0 + k * zstride, A.w, cd[k], p.img[U.w], B.w != 0, hi, hj, hk);
+        else
+          st[k].image(p, n0 + k * zstride, A.w, cd[k], spin_velocity(p.img[U.w], hi, hj, hk));
       }
-    } else {
+    } else if constexpr (!F64) {
       const float4 nv = make_float4(0.f, __int_as_float(U.x), __int_as_float(U.y),
                                     __int_as_float(U.z));
 #pragma unroll
@@ -869,15 +784,13 @@ cudaError_t launch_map(const MapParams& p, cudaStream_t st, cudaStream_t aux, cu
     if ((e = cudaEventRecord(join, aux)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(st, join, 0)) != cudaSuccess) return e;
   }
-  dim3 block(p.cb[0], p.cb[1], p.cb[2]);
-  dim3 cells((unsigned)p.C[0], (unsigned)p.C[1], (unsigned)p.C[2]);
-  if (p.write32) {
-    constexpr int NPT = 2;  // nodes per thread along z
-    dim3 part(p.cb[0], p.cb[1], (p.cb[2] + NPT - 1) / NPT);
-    node_apply32_kernel<NPT><<<cells, part, 0, st>>>(p);
-  } else {
-    node_apply_kernel<<<cells, block, 0, st>>>(p);
-  }
+  constexpr int NPT = 2;  // nodes per thread along z
+  const dim3 cells((unsigned)p.C[0], (unsigned)p.C[1], (unsigned)p.C[2]);
+  const dim3 part(p.cb[0], p.cb[1], (p.cb[2] + NPT - 1) / NPT);
+  if (p.write32)
+    node_apply_kernel<false, NPT><<<cells, part, 0, st>>>(p);
+  else
+    node_apply_kernel<true, NPT><<<cells, part, 0, st>>>(p);
   return cudaGetLastError();
 }
 
