@@ -25,6 +25,8 @@
 // (deterministic run to run).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "lbmpsm_internal.cuh"
 #include "solid_fraction.cuh"
 
@@ -420,11 +422,17 @@ constexpr int SFS_THREADS = 128;  // shell counting: persistent warps
 // one per lane, and the warp walks their nodes 32 at a time (consecutive lanes
 // on consecutive nodes of a row).
 //
-// With many images one block of two warps each, 32 rows a group (2260 images
-// of diameter 12: one wave); with few, an image's groups of 8 rows are dealt
-// to SFC_PARTS blocks (one image of diameter 16 by one block: 30 us).
+// With many images 32 rows a group: one block an image, or, for fewer than four
+// images a multiprocessor, as many as keep 16 blocks of two warps on each, up to
+// eight (classify_parts; 284 images: 8 us less a step.  About 900 images in three
+// blocks each: one workload 5 us a step faster, another 1.3 slower, so one).
+// With few images, groups of 8 rows are dealt to SFC_PARTS blocks (one image of
+// diameter 16 by one block: 30 us).
 constexpr int SFC_QW = 256;  // per-warp queue of shell nodes
 constexpr int SFC_PARTS = 16;
+static unsigned classify_parts(int n, int sm_count) {
+  return n < 4 * sm_count ? (unsigned)std::min(SFC_PARTS / 2, 16 * sm_count / n) : 1u;
+}
 template <int ROWS>
 __global__ void __launch_bounds__(SFC_THREADS) sf_classify_kernel(MapParams p) {
   const Img& im = p.img[blockIdx.x];
@@ -778,7 +786,7 @@ cudaError_t launch_map(const MapParams& p, cudaStream_t st, cudaStream_t aux, cu
   if (few_images(p.n, p.sm_count))
     sf_classify_kernel<8><<<dim3((unsigned)p.n, SFC_PARTS), SFC_THREADS, 0, st>>>(p);
   else
-    sf_classify_kernel<32><<<p.n, SFC_THREADS, 0, st>>>(p);
+    sf_classify_kernel<32><<<dim3((unsigned)p.n, classify_parts(p.n, p.sm_count)), SFC_THREADS, 0, st>>>(p);
   sf_shell_kernel<<<p.sm_count * 8, SFS_THREADS, 0, st>>>(p);
   if (two) {
     if ((e = cudaEventRecord(join, aux)) != cudaSuccess) return e;
