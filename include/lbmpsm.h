@@ -341,7 +341,7 @@ void lbmpsm_group_destroy(lbmpsm_group* g);
  *
  * lbmpsm_adjoint_drag: reverse sweep.  The state before every
  * checkpoint_every-th step is kept in HBM; the reverse pass recomputes each
- * segment from its checkpoint.  Device memory: (nsteps/checkpoint_every +
+ * segment but the last from its checkpoint.  Device memory: (nsteps/checkpoint_every +
  * checkpoint_every + 1) population arrays (FP64, Q per node).  Outputs (any
  * may be NULL except dJ_dx when n > 0): J; dJ/dtau; dJ/dFext[3]; dJ/dx[3n]
  * per image row; the total drag along direction of every step [nsteps].

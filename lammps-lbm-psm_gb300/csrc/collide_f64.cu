@@ -292,10 +292,11 @@ __device__ __forceinline__ void collide_dirs(NodeCols<L, FORCE>& s, int t, const
 
 // One node of the FP64 collide + A-A stream step.
 //
-// Bound by the FP64 pipe (1.68 operations per clock and multiprocessor, the
-// memory system at a few per cent), so: sums near rest run on the integer
-// units beside it (fixed_f64.cuh), what directions share is formed once
-// (pair_feq), three quotients share one reciprocal (div3), the body force is
+// Bound by the FP64 pipe (1.68 operations per clock and multiprocessor) and,
+// with the work split, as much by the integer units (both 50 to 65% busy; DRAM
+// 11%), so: sums and equilibria near rest run on the integer units
+// (fixed_f64.cuh), what directions share is formed once (pair_diff), three
+// quotients share one reciprocal (div3), the body force is
 // a template argument, and a warp takes the plain loop when none of its nodes
 // is a PSM node, the one-slot loop when none holds two particles -- an unused
 // slot has B = 0 and adds zeros, and a node without any has 1 - B = 1, so the
