@@ -1859,7 +1859,11 @@ AdjParams adj_params(const lbmpsm_handle* h, const AdjNodes& an, double* part,
   p.weighting = h->opt.psm_weighting;
   p.an = an;
   p.part = part;
-  for (int d = 0; d < 3; ++d) p.d[d] = direction[d];
+  for (int d = 0; d < 3; ++d) {
+    p.d[d] = direction[d];
+    p.F3[d] = 3.0 * p.bp.F[d];
+    p.F9[d] = 9.0 * p.bp.F[d];
+  }
   return p;
 }
 

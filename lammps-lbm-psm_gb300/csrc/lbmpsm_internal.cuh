@@ -433,6 +433,7 @@ struct AdjParams {
   double* lout;         // adjoint: lambda of this step; tangent: the next step's tangent
   double c;             // objective weight of this step
   double d[3];          // drag direction
+  double F3[3], F9[3];  // 3 F and 9 F (lattice units)
   double* part;         // per-block partial sums, ADJ_PART per block
   double domega, dtau, dF[3];  // tangent direction (lattice units)
 };
