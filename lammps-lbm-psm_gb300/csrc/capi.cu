@@ -2083,7 +2083,10 @@ int lbmpsm_tangent_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   const double omega_lb = h->boxes[0].omega;
   p.dtau = dtau;
   p.domega = -omega_lb * omega_lb * dtau;
-  for (int d = 0; d < 3; ++d) p.dF[d] = dFext ? dFext[d] / h->volumeForceFactor : 0.0;
+  for (int d = 0; d < 3; ++d) {
+    p.dF[d] = dFext ? dFext[d] / h->volumeForceFactor : 0.0;
+    p.force[d] = (1.0 - 0.5 * omega_lb) * p.dF[d] - 0.5 * p.domega * p.bp.F[d];
+  }
   const double cwin = h->forceFactor / (double)(t1 - t0 + 1);
   const long long ts = h->t;
   int cur = 0;

@@ -436,6 +436,7 @@ struct AdjParams {
   double F3[3], F9[3];  // 3 F and 9 F (lattice units)
   double* part;         // per-block partial sums, ADJ_PART per block
   double domega, dtau, dF[3];  // tangent direction (lattice units)
+  double force[3];             // (1 - omega/2) dF - domega/2 F
 };
 constexpr int ADJ_PART = 5;  // d/domega, d/dtau through B, d/dF[3] (tangent: dJ in [0])
 
