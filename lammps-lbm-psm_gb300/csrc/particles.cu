@@ -944,6 +944,10 @@ static __device__ __forceinline__ void reduce_image(const ReduceParams& p) {
   // nodes in the same order whatever U)
   constexpr int U = C == 1 ? (F64 ? 1 : 2) : (F64 ? 4 : 8);
   __shared__ Pair part[RED_MAX_GROUPS][12];
+  // the first block's shared memory may be written once every block of the
+  // cluster is known to run: all arrive here and wait before their groups, so
+  // that the loads of the image lie between
+  if (C > 1) cooperative_groups::this_cluster().barrier_arrive();
   const int ip = C == 1 ? (int)blockIdx.x : (int)blockIdx.x / C;
   const int rank = C == 1 ? 0 : (int)blockIdx.x % C;
   const Geom& g = p.g;
@@ -959,6 +963,7 @@ static __device__ __forceinline__ void reduce_image(const ReduceParams& p) {
   const double xl0 = F64 ? bx.xl[0] : 0.0;
   const float rem0 = bx.rP2f * 1.0001f + 0.01f;
   Pair total = S::zero();  // thread k < 12 of the first block: sum k
+  if (C > 1) cooperative_groups::this_cluster().barrier_wait();
   for (int g0 = 0; g0 < G || g0 == 0; g0 += RED_MAX_GROUPS) {
     const int gend = min(G, g0 + RED_MAX_GROUPS);
     for (int gi = g0 + warp * C + rank; gi < gend; gi += C * NW) {
