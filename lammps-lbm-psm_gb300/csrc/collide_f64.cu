@@ -378,7 +378,8 @@ __device__ __forceinline__ void collide_f64_node(NodeCols<L, FORCE>& s, const Co
   nd.uz = u[2];
   nd.axis = -1;
   if (has_force) {
-    const bool z0 = is_zero(bp.F[0]), z1 = is_zero(bp.F[1]), z2 = is_zero(bp.F[2]) || L::DIM == 2;
+    // (an out-of-plane force has its part in D2Q9 too, through u_z)
+    const bool z0 = is_zero(bp.F[0]), z1 = is_zero(bp.F[1]), z2 = is_zero(bp.F[2]);
     if (z1 && z2) nd.axis = 0;
     if (z0 && z2) nd.axis = 1;
     if (L::DIM == 3 && z0 && z1) nd.axis = 2;
