@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/lbmpsm.h"
+#include "host_access.h"
 #include "lbmpsm_internal.cuh"
 
 using namespace lbmpsm;
@@ -1485,7 +1486,7 @@ int lbmpsm_export_fields(lbmpsm_handle* h, int as_double, double B0, double rho0
   const long long base = box_base(h);
   const size_t npts = (size_t)(g.L[0] - 2) * (g.L[1] - 2) * (g.dim == 3 ? g.L[2] - 2 : 1);
   const size_t es = as_double ? 8 : 4;
-  if (h->host_direct) {  // the kernel writes the caller's arrays
+  if (in_place(h->host_direct, es, {solid, rho, u})) {  // the kernel writes the caller's arrays
     if (solid) prefault(solid, es * npts);
     if (rho) prefault(rho, es * npts);
     if (u) prefault(u, 3 * es * npts);
@@ -1515,7 +1516,7 @@ int lbmpsm_get_populations(lbmpsm_handle* h, double* f) {
   CUDA_TRY(h, cudaSetDevice(h->device));
   const Geom g = box_geom(h);
   const size_t cnt = (size_t)g.L[0] * g.L[1] * g.L[2] * g.Q;
-  if (h->host_direct) {  // the kernel writes the caller's array
+  if (in_place(h->host_direct, sizeof(double), {f})) {  // the kernel writes the caller's array
     prefault(f, sizeof(double) * cnt);
     CUDA_TRY(h, launch_get_populations(g, box_f(h), h->opt.storage, (h->t % 2 == 0) ? 1 : 0, h->scale16,
                                        f, h->stream));
@@ -1538,7 +1539,7 @@ int lbmpsm_set_populations(lbmpsm_handle* h, const double* f) {
   CUDA_TRY(h, cudaSetDevice(h->device));
   const Geom g = box_geom(h);
   const size_t cnt = (size_t)g.L[0] * g.L[1] * g.L[2] * g.Q;
-  if (h->host_direct) {  // the kernel reads the caller's array
+  if (in_place(h->host_direct, sizeof(double), {f})) {  // the kernel reads the caller's array
     CUDA_TRY(h, launch_set_populations(g, box_f(h), h->opt.storage, (h->t % 2 == 0) ? 1 : 0, h->scale16,
                                        f, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
