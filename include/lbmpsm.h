@@ -224,8 +224,8 @@ void* lbmpsm_stream(lbmpsm_handle* h);
  * a NULL handle.  Both give the same results bit for bit.  Single-box
  * handles only: lbmpsm_step_batch always stages.  With 1, lbmpsm_get_populations,
  * lbmpsm_set_populations and lbmpsm_export_fields also work on the caller's
- * arrays, unless one of the call's is not aligned to its elements: the call
- * then stages all of them. */
+ * arrays.  A call one of whose arrays is not aligned to its elements stages
+ * all of them. */
 int lbmpsm_host_direct(const lbmpsm_handle* h);
 
 /* Run nsteps coupling steps with the particle images already on the device

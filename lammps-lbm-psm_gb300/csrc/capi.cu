@@ -1297,7 +1297,8 @@ int step_impl(lbmpsm_handle* h, int n, const int* box, const int* tag, const dou
     return fail(h, LBMPSM_ERR_ARG, "NULL particle array");
   int rc = maybe_tune(h);
   if (rc) return rc;
-  if (h->host_direct && !box && h->nbox == 1 && n > 0) {
+  if (!box && h->nbox == 1 && n > 0 && in_place(h->host_direct, sizeof(int), {tag}) &&
+      in_place(h->host_direct, sizeof(double), {x, v, omega, radius, fh, th, stresslet})) {
     // no staging: the device-step graph on the caller's host arrays
     CUDA_TRY(h, cudaSetDevice(h->device));
     double rmax = 0.0;

@@ -26,9 +26,10 @@ def test_in_place_needs_aligned_arrays(tmp_path):
         assert answers == ("11110" if ok else "00010"), (element, off)
 
 
-@pytest.mark.parametrize("call", ["lbmpsm_export_fields", "lbmpsm_get_populations", "lbmpsm_set_populations"])
+@pytest.mark.parametrize("call", ["lbmpsm_export_fields", "lbmpsm_get_populations", "lbmpsm_set_populations",
+                                  "step_impl"])
 def test_every_call_asks(call):
     src = open(os.path.join(CSRC, "capi.cu")).read()
     body = re.search(r"\nint %s\(.*?\n}\n" % call, src, re.S).group(0)
-    assert re.search(r"if \(in_place\(h->host_direct,", body)
+    assert re.search(r"if \([^{]*in_place\(h->host_direct,", body)
     assert "if (h->host_direct" not in body

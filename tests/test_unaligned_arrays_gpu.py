@@ -54,3 +54,27 @@ def test_fields(off, as_double, which):
     a._check(a.lib.lbmpsm_export_fields(a.h, int(as_double), 0.5, 2.0, 3.0, *[g.ctypes.data for g in got]))
     for p, q in zip(want, got):
         assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("storage", ["fp64", "fp32"])
+@pytest.mark.parametrize("which", range(6))
+def test_step(storage, which):
+    """Image arrays and outputs at odd offsets, some steps aligned in between."""
+    c = cases.CASES["shear_3d"]
+    a, b = cases.GpuBackend(c, storage).lat, cases.GpuBackend(c, storage).lat
+    tag, x, v, w, r = cases.initial_particles(c)
+    for step in range(8):
+        g = cases.images(c, tag, x, v, w, r, cases.product_make_ghosts)
+        arrays = [np.ascontiguousarray(g[k]) for k in ("tag", "x", "v", "omega", "radius")]
+        want = a.step(*arrays)
+        out = np.empty(12 * len(arrays[0]))
+        if step not in (1, 5):
+            if which < 5:
+                arrays[which] = unaligned(arrays[which], 2 if which == 0 else 4)
+            else:
+                out = unaligned(out, 4)
+        got = b.step(*arrays, out=out)
+        for p, q in zip(want, got):
+            assert np.array_equal(p, q)
+        assert np.array_equal(a.populations(), b.populations())
+        x = cases.advance(c, x, v)
