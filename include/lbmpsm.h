@@ -285,11 +285,13 @@ int lbmpsm_export_fields_static(lbmpsm_handle* h, int as_double, double B0, doub
  * lbmpsm_run_fixed would (each with the images it holds from its last step,
  * each with its boundary condition), with one step of all members captured
  * once per A-A parity into a single CUDA graph whose branches run
- * concurrently, so that every step is one graph launch.  Members must be on
- * one device and at the same step parity; a member with a macro-field store
- * pending is rejected (LBMPSM_ERR_STATE).  The group's work is ordered after
- * the members' earlier work and before their later work.  Destroy the group
- * before its members. */
+ * concurrently, so that every step is one graph launch.  As there, a call of
+ * several steps waits after its first ones (three times at most) to see whether
+ * every member's table has settled; from then on its steps run without the maps.
+ * Members must be on one device and at the same step parity; a member with a
+ * macro-field store pending is rejected (LBMPSM_ERR_STATE).  The group's work is
+ * ordered after the members' earlier work and before their later work.  Destroy
+ * the group before its members. */
 typedef struct lbmpsm_group lbmpsm_group;
 int lbmpsm_group_create(lbmpsm_handle* const* handles, int count, lbmpsm_group** out);
 /* When every member is 3-D and periodic on every axis, the members share
@@ -308,10 +310,11 @@ int lbmpsm_group_run_fixed(lbmpsm_group* g, int nsteps);
 int lbmpsm_group_collide_launches(const lbmpsm_group* g);
 /* The group's tuner: the first lbmpsm_group_run_fixed call with at least 8
  * steps, on members that qualify for one collide launch, runs two steps of
- * each plan untimed (capturing their graphs) and two timed, then keeps the
- * faster plan for the rest of the group's life (both give the same results
- * bit for bit).  ms[0] = per-member launches, ms[1] = one launch, in ms per
- * step (-1: not timed).  LBMPSM_GROUP_FUSE=0 / =1 fixes the plan instead. */
+ * each plan untimed (capturing their graphs) and two timed, all four timed ones
+ * with the maps or all without, then keeps the faster plan for the rest of the
+ * group's life (both give the same results bit for bit).  ms[0] = per-member
+ * launches, ms[1] = one launch, in ms per step (-1: not timed).
+ * LBMPSM_GROUP_FUSE=0 / =1 fixes the plan instead. */
 int lbmpsm_group_tune_ms(const lbmpsm_group* g, float* ms);
 void* lbmpsm_group_stream(lbmpsm_group* g); /* the cudaStream_t the group's graphs run on */
 const char* lbmpsm_group_last_error(const lbmpsm_group* g);

@@ -40,6 +40,7 @@ def _deps(unit: str) -> list[str]:
             os.path.join(CSRC, "solid_fraction.cuh"),
             os.path.join(CSRC, "fixed_f64.cuh"),
             os.path.join(CSRC, "host_access.h"),
+            os.path.join(CSRC, "held_run.h"),
             os.path.join(ROOT, "include", "lbmpsm.h")]
 
 

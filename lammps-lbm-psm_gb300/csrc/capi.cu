@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/lbmpsm.h"
+#include "held_run.h"
 #include "host_access.h"
 #include "lbmpsm_internal.cuh"
 
@@ -679,9 +680,6 @@ int map_settled(lbmpsm_handle* h, cudaStream_t st, bool& settled) {
   settled = changed == 0;
   return LBMPSM_OK;
 }
-// Steps of a run after which it is asked (a table that particles have just
-// moved over settles with the second or third map).
-bool ask_settled(int step) { return step >= 1 && step <= 3; }
 
 int read_status(lbmpsm_handle* h) {
   int st = 0;
@@ -1638,19 +1636,20 @@ int lbmpsm_run_fixed(lbmpsm_handle* h, int nsteps) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(h, cudaStreamIsCapturing(h->stream, &cs));
   const bool may_settle = n > 0 && cs == cudaStreamCaptureStatusNone;
-  bool settled = false;
+  SettleQuestions q;
   for (int s = 0; s < nsteps; ++s) {
     const int par = (int)(h->t & 1);
-    if (may_settle && !settled && ask_settled(s) && nsteps - s >= 4) {
-      const int rc = map_settled(h, h->stream, settled);
+    if (may_settle && q.due(s, nsteps - s)) {
+      ++q.asked;
+      const int rc = map_settled(h, h->stream, q.settled);
       if (rc) return rc;
     }
-    cudaGraphExec_t* const exec = settled ? h->sexec : h->gexec;
+    cudaGraphExec_t* const exec = q.settled ? h->sexec : h->gexec;
     if (!exec[par]) {
       cudaGraph_t graph = nullptr;
       CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
       const long long t0 = h->t;
-      int rc = enqueue_step(h, n, use_bc, !settled, true);
+      int rc = enqueue_step(h, n, use_bc, !q.settled, true);
       cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
       h->t = t0;  // captured, not run
       if (rc) {
@@ -1986,21 +1985,22 @@ int lbmpsm_adjoint_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   auto first = [&](int seg) { return seg == 0 ? 1 : T - (nseg - seg) * K + 1; };
   // forward pass: the ordinary steps, a checkpoint before each segment's first
   const long long ts = h->t;
-  bool settled = false;
+  SettleQuestions q;
   for (int t = 1, seg = 0; t <= T; ++t) {
     if (seg < nseg && t == first(seg))
       CUDA_TRY(h, cudaMemcpyAsync(ckpt[(size_t)seg++], h->f, state, cudaMemcpyDeviceToDevice, h->stream));
     else if (seg == nseg)
       CUDA_TRY(h, cudaMemcpyAsync(store[(size_t)(t - first(nseg - 1) - 1)], h->f, state,
                                   cudaMemcpyDeviceToDevice, h->stream));
-    rc = enqueue_step(h, n, false, !settled, true);
+    rc = enqueue_step(h, n, false, !q.settled, true);
     if (rc) return rc;
     if (t == 1) {
       rc = adj_entries(h, an, n, centre_step);
       if (rc) return rc;
     }
-    if (n > 0 && !settled && ask_settled(t) && t < T) {
-      rc = map_settled(h, h->stream, settled);
+    if (n > 0 && q.due(t, T - t, 1)) {
+      ++q.asked;
+      rc = map_settled(h, h->stream, q.settled);
       if (rc) return rc;
     }
     if (n > 0)
@@ -2102,7 +2102,7 @@ int lbmpsm_tangent_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
   const double cwin = h->forceFactor / (double)(t1 - t0 + 1);
   const long long ts = h->t;
   int cur = 0;
-  bool settled = false;
+  SettleQuestions q;
   for (int t = 1; t <= T; ++t) {
     // the tangent step reads the state before this step's collide; the table
     // it needs exists after the first map, so step 1 runs from a copy
@@ -2116,10 +2116,11 @@ int lbmpsm_tangent_drag(lbmpsm_handle* h, int n, const int* tag, const double* x
       CUDA_TRY(h, launch_adj_step(p, 1, h->stream));
       cur ^= 1;
     }
-    rc = enqueue_step(h, n, false, !settled, true);
+    rc = enqueue_step(h, n, false, !q.settled, true);
     if (rc) return rc;
-    if (n > 0 && !settled && ask_settled(t) && t < T) {
-      rc = map_settled(h, h->stream, settled);
+    if (n > 0 && q.due(t, T - t, 1)) {
+      ++q.asked;
+      rc = map_settled(h, h->stream, q.settled);
       if (rc) return rc;
     }
     if (t == 1) {
@@ -2366,6 +2367,52 @@ int group_step(lbmpsm_group* g, bool map) {
   for (lbmpsm_handle* h : g->hs) h->t += 1;
   return LBMPSM_OK;
 }
+
+// The calls that run_group_steps orders.
+struct GroupOps {
+  lbmpsm_group* g;
+  int ask(bool& settled) {
+    settled = true;
+    for (size_t i = 0; settled && i < g->hs.size(); ++i) {
+      if (g->hs[i]->last_n == 0) continue;
+      const int rc = map_settled(g->hs[i], g->stream, settled);
+      if (rc) return gfail(g, rc, g->hs[i]->err);
+    }
+    return LBMPSM_OK;
+  }
+  int step(bool map) { return group_step(g, map); }
+  int plan(int which) {
+    group_drop(g);
+    g->plan_pref = which;
+    return LBMPSM_OK;
+  }
+  int ready(bool map) {
+    for (int par = 0; par < 2; ++par) {
+      cudaGraphExec_t& exec = (map ? g->gexec : g->sexec)[par];
+      if (exec) continue;
+      const int rc = group_capture(g, par, map);
+      if (rc) return rc;
+      GROUP_TRY(g, cudaGraphUpload(exec, g->stream));
+    }
+    return LBMPSM_OK;
+  }
+  int start() {
+    GROUP_TRY(g, cudaEventRecord(g->t0, g->stream));
+    return LBMPSM_OK;
+  }
+  int stop(int which) {
+    GROUP_TRY(g, cudaEventRecord(g->t1, g->stream));
+    GROUP_TRY(g, cudaEventSynchronize(g->t1));
+    float ms = 0.f;
+    GROUP_TRY(g, cudaEventElapsedTime(&ms, g->t0, g->t1));
+    g->tune_ms[which] = ms / 2;
+    return LBMPSM_OK;
+  }
+  int choose() {
+    const int best = g->tune_ms[1] <= g->tune_ms[0] ? 1 : 0;
+    return best == g->plan_pref ? LBMPSM_OK : plan(best);
+  }
+};
 }  // namespace
 
 extern "C" {
@@ -2467,63 +2514,17 @@ int lbmpsm_group_run_fixed(lbmpsm_group* g, int nsteps) {
     GROUP_TRY(g, cudaEventRecord(g->join[i], g->hs[i]->stream));
     GROUP_TRY(g, cudaStreamWaitEvent(g->stream, g->join[i], 0));
   }
-  // one step; after the first ones, whether every member's table is settled
-  // (map_settled: from then on the steps run without the maps)
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   GROUP_TRY(g, cudaStreamIsCapturing(g->stream, &cs));
-  bool settled = false;
-  int done = 0;
-  auto step = [&]() -> int {
-    if (!settled && cs == cudaStreamCaptureStatusNone && ask_settled(done) && nsteps >= 4) {
-      settled = true;
-      for (size_t i = 0; settled && i < m; ++i) {
-        if (g->hs[i]->last_n == 0) continue;
-        const int rc = map_settled(g->hs[i], g->stream, settled);
-        if (rc) return gfail(g, rc, g->hs[i]->err);
-      }
-    }
-    const int rc = group_step(g, !settled);
-    ++done;
-    --nsteps;
-    return rc;
-  };
   // the group's tuner: with at least 8 steps to run and members that qualify
   // for one collide launch, time two steps of each plan (after two untimed
   // steps that capture its graphs) and keep the faster
   const char* fenv = std::getenv("LBMPSM_GROUP_FUSE");
-  if (!g->tuned && nsteps >= 8 && !fenv && group_fusable(g)) {
-    g->tuned = true;
-    for (int plan = 1; plan >= 0; --plan) {
-      group_drop(g);
-      g->plan_pref = plan;
-      for (int k = 0; k < 2; ++k) {
-        const int rc = step();
-        if (rc) return rc;
-      }
-      for (int par = 0; par < 2; ++par) {  // no capture among the timed steps
-        if ((settled ? g->sexec : g->gexec)[par]) continue;
-        const int rc = group_capture(g, par, !settled);
-        if (rc) return rc;
-      }
-      GROUP_TRY(g, cudaEventRecord(g->t0, g->stream));
-      for (int k = 0; k < 2; ++k) {
-        const int rc = step();
-        if (rc) return rc;
-      }
-      GROUP_TRY(g, cudaEventRecord(g->t1, g->stream));
-      GROUP_TRY(g, cudaEventSynchronize(g->t1));
-      float ms = 0.f;
-      GROUP_TRY(g, cudaEventElapsedTime(&ms, g->t0, g->t1));
-      g->tune_ms[plan] = ms / 2;
-    }
-    const int best = g->tune_ms[1] <= g->tune_ms[0] ? 1 : 0;
-    if (best != g->plan_pref) group_drop(g);
-    g->plan_pref = best;
-  }
-  while (nsteps > 0) {
-    const int rc = step();
-    if (rc) return rc;
-  }
+  const bool tune = !g->tuned && nsteps >= 8 && !fenv && group_fusable(g);
+  if (tune) g->tuned = true;
+  GroupOps ops{g};
+  const int rc = run_group_steps(ops, nsteps, cs == cudaStreamCaptureStatusNone, tune);
+  if (rc) return rc;
   // the members' later work is ordered after the group's
   GROUP_TRY(g, cudaEventRecord(g->done, g->stream));
   for (size_t i = 0; i < m; ++i) GROUP_TRY(g, cudaStreamWaitEvent(g->hs[i]->stream, g->done, 0));
