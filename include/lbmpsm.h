@@ -76,8 +76,11 @@ extern "C" {
  * step, while the stream is being captured; the default shape is kept if the
  * allocation fails).  The candidates give bit-identical results.  DEFAULT:
  * the 3-stage pipeline, untimed.  The environment variable LBMPSM_PIPE_STAGES
- * (2..5 stages, or 0 = the direct kernel) overrides both.  Rows longer than 256
- * nodes have one shape each, chosen by their length, and are not timed. */
+ * (2..5 stages, or 0 = the direct kernel, which rounds |u_s|^2 in another order)
+ * overrides both.  Lattices of many short rows take several rows a tile with two
+ * or three stages, one with four or five, which the tuner does not time there.
+ * Rows longer than 256 nodes have one shape each, chosen by their length, and are
+ * not timed; they round as the direct kernel does. */
 #define LBMPSM_TUNE_AUTO 0
 #define LBMPSM_TUNE_DEFAULT 1
 

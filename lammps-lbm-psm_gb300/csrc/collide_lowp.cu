@@ -38,14 +38,14 @@ cudaError_t launch_collide_multi(const MultiCollide& mc, int storage, int odd, c
 
 // The project's autotuner for the FP32/FP16 collide: every candidate launch
 // shape -- the row pipeline with 3, 2, 4 or 5 stages, each at the blocks per
-// multiprocessor its shared memory and registers allow -- runs a few even/odd
-// step pairs on p.f (a scratch copy of the populations), timed with CUDA
-// events on the stream; the fastest is kept.  The candidates are one template
+// multiprocessor its shared memory and registers allow -- runs even/odd step
+// pairs on p.f (a scratch copy of the populations), timed with CUDA events on
+// the stream; the fastest is kept.  The candidates are one template
 // (only the stage count and the launch bounds differ), so they round alike
 // and the choice changes speed only, never results.  The direct kernel rounds
 // |u_s|^2 in another order and is not a candidate.
 //
-// One pair untimed, then one timed, three where a pair is shorter than 200 us
+// A pair untimed, then one timed, or three where a pair is shorter than 200 us
 // or so (a rate of 3 TB/s assumed).
 static const int cand[LBMPSM_TUNE_CANDIDATES] = {3, 2, 4, 5};
 
@@ -53,8 +53,10 @@ int tune_shapes(const Geom& g, int storage, int sm_count, PipeConfig (&shape)[LB
   int n = 0;
   for (int k = 0; k < LBMPSM_TUNE_CANDIDATES; ++k) {
     PipeConfig& c = shape[k];
-    // (a long row has one shape whatever the stages asked for)
-    if (prepare_collide_lowp(g, storage, sm_count, cand[k], &c) != cudaSuccess || c.stages != cand[k])
+    // (a long row has one shape whatever the stages asked for; where tiles hold
+    // several rows, one row a tile is the slower shape and not timed)
+    if (prepare_collide_lowp(g, storage, sm_count, cand[k], &c) != cudaSuccess || c.stages != cand[k] ||
+        c.k < shape[0].k)
       c = PipeConfig{};
     if (c.grid > 0) ++n;
   }

@@ -1181,8 +1181,8 @@ static cudaError_t prepare_lowp(const Geom& g, int sm_count, int stages, PipeCon
   *cfg = PipeConfig{};
   if (stages == 0) return cudaSuccess;
   if (g.S[0] > PIPE_CONSUMERS && (stages = long_row_stages<L, T>(g, sm_count)) == 0) return cudaSuccess;
-  const int k = tile_rows(g, (sizeof(T) == 2 ? 4 : 3) * sm_count);
-  if (k > 1 && stages > 3) return cudaSuccess;
+  // (several rows a tile have two or three stages; with more, one row a tile)
+  const int k = stages > 3 ? 1 : tile_rows(g, (sizeof(T) == 2 ? 4 : 3) * sm_count);
   return with_shape<T>(g, stages, k, [&](auto nst, auto minb, auto mode) {
     return pipe_prepare<L, T, nst, minb, mode>(g, sm_count, k, cfg);
   });
