@@ -11,9 +11,9 @@
 // is rounded to 53 significant bits, ties to even, as the IEEE operation it
 // stands for.  Products by the constants 3, 4.5 and 1.5 and of a density with a
 // factor are formed the same way.  Every function states the range it needs;
-// the caller checks the ranges (populations in [2^-7, 1), densities above 0.9
-// and below 2, velocity components below 5/64) and takes the FP64 expressions
-// otherwise.  A suspension whose spheres move at 0.04 stays inside.
+// the ranges are checked (populations and density in macro_sums, velocity
+// components below 5/64 by the caller) and the FP64 expressions taken otherwise.
+// A suspension whose spheres move at 0.04 stays inside.
 //
 // Host compilable: the functions are compared with IEEE arithmetic on the CPU.
 #pragma once
@@ -181,7 +181,10 @@ LBMPSM_HD u64 to62(double x) {
 
 // the product of r (units of 2^-64) and s (units of 2^-62), rounded to 53 bits,
 // in units of 2^-62: from 2^-7 to 2, so that at least three bits of the unit
-// lie below the last place
+// lie below the last place.  (An equilibrium rho*w*factor is at least 0.0094:
+// macro_sums lets densities of 0.609375 (D3Q19) and 0.5546875 (D2Q9) through at
+// the lowest, w is 1/36 at the lowest, and with velocity components below 5/64 a
+// factor is above 0.613 = 1 - 3 (5/32) + 4.5 (5/32)^2 - 1.5 * 3 (5/64)^2.)
 LBMPSM_HD u64 product62(u64 r, u64 s) {
   const unsigned __int128 x = (unsigned __int128)r * s;
   const u64 t = (u64)(x >> 64) | ((u64)x != 0 ? 1ull : 0ull);
@@ -213,7 +216,9 @@ LBMPSM_HD double difference62(u64 a, u64 b) {
 // component along a.  Returns whether every range held (else the outputs are
 // not to be used): populations in [2^-7, 1), the sum of the first two (D3Q19:
 // the first two in [1/4, 1/2), the first three below 1/2; the first five) at
-// least 1/2, the density below 2, the partial sums of j below 1/4.
+// least 1/2, the density below 2, the partial sums of j below 1/4.  With the other
+// populations at 2^-7 at least, the density is 1/2 + 14/128 = 0.609375 (D3Q19) or
+// 1/2 + 7/128 = 0.5546875 (D2Q9) at the lowest.
 template <class L>
 LBMPSM_HD bool macro_sums(const double* f, double& rho, double (&j)[3]) {
   constexpr int Q = L::Q;
