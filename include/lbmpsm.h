@@ -325,9 +325,10 @@ void lbmpsm_group_destroy(lbmpsm_group* g);
 
 /* Sensitivities of the time-averaged drag (the reference has
  * no adjoint; the forward step is lbmpsm_step's).  Both calls run nsteps
- * ordinary coupling steps with one fixed set of particle images -- exactly
- * the launches of nsteps lbmpsm_step calls with these arrays, so the lattice
- * ends where those calls leave it -- and differentiate
+ * ordinary coupling steps with one fixed set of particle images -- the
+ * launches of nsteps lbmpsm_step calls with these arrays, less the maps once
+ * the particle table has settled (as in lbmpsm_run_fixed), so the lattice ends
+ * where those calls leave it -- and differentiate
  *
  *   J = 1/M * sum_{t=t0..t1} sum_images  direction . F_image(t),  M = t1-t0+1,
  *
