@@ -458,7 +458,7 @@ __device__ __forceinline__ bool mbar_wait_abortable(unsigned bar, unsigned phase
 // Warp-specialised pipeline of the collide / A-A stream step.  A persistent
 // grid; every block walks its tiles t, t + G, t + 2G, ... through NST
 // shared-memory stages of Q populations per node.  A tile is
-//   ONE_ROW, ONE_SHORT_ROW: one x-row of up to 256, 128 nodes;
+//   ONE_ROW, ONE_MID_ROW, ONE_SHORT_ROW: one x-row of up to 256, 192, 128 nodes;
 //   SOME_ROWS: p.pipe.k consecutive rows of a plane, as many as fit 256 nodes,
 //     so that short rows fill the block and its copies (rows of 32 nodes one at
 //     a time moved 128 bytes a copy and kept one consumer warp a block: the
@@ -482,11 +482,15 @@ __device__ __forceinline__ bool mbar_wait_abortable(unsigned bar, unsigned phase
 // (after p.full_wait_limit polls) raise a shared abort flag, which ends the
 // producer's wait for their signal at once; the producer then waits, with
 // its own long limit, only for the loads it has issued.
-enum PipeMode { ONE_ROW, ONE_SHORT_ROW, SOME_ROWS, LONG_ROW };
+enum PipeMode { ONE_ROW, ONE_MID_ROW, ONE_SHORT_ROW, SOME_ROWS, LONG_ROW };
 // Staged nodes of one direction: fixed (but for long rows), so that the
 // consumers' 38 shared-memory addresses a node are two or three registers and
-// constants.
-__host__ __device__ constexpr int pipe_stride(int mode) { return mode == LONG_ROW ? 0 : (mode == ONE_SHORT_ROW ? 128 : 256); }
+// constants.  Rows of up to 192 nodes have their own, which leaves room for a
+// fourth block of three FP32 stages (160 x 96 x 96: 40.2 us a step, at the
+// distance of 256 nodes 42.8; 144 x 200 x 200: 143.6 and 155.5).
+__host__ __device__ constexpr int pipe_stride(int mode) {
+  return mode == LONG_ROW ? 0 : (mode == ONE_SHORT_ROW ? 128 : (mode == ONE_MID_ROW ? 192 : 256));
+}
 template <class L, typename T, bool ODD, bool FORCE, int NST, int MINB, int MODE>
 __global__ void __launch_bounds__(PIPE_CONSUMERS + 32, MINB) collide_pipe_kernel(CollideParams p) {
   static_assert(NST >= 2, "stages");
@@ -1140,6 +1144,7 @@ static cudaError_t with_shape(const Geom& g, int stages, int k, Fn fn) {
   typedef std::integral_constant<int, 5> I5;
   typedef std::integral_constant<int, B> IB;
   typedef std::integral_constant<int, ONE_ROW> One;
+  typedef std::integral_constant<int, ONE_MID_ROW> Mid;
   typedef std::integral_constant<int, ONE_SHORT_ROW> Short;
   typedef std::integral_constant<int, SOME_ROWS> Some;
   typedef std::integral_constant<int, LONG_ROW> Long;
@@ -1150,6 +1155,12 @@ static cudaError_t with_shape(const Geom& g, int stages, int k, Fn fn) {
     case 4: return fn(I4(), I2(), Short());
     case 5: return fn(I5(), I2(), Short());
     default: return fn(I3(), IB(), Short());
+  }
+  if (g.P0 <= pipe_stride(ONE_MID_ROW)) switch (stages) {
+    case 2: return fn(I2(), IB(), Mid());
+    case 4: return fn(I4(), I2(), Mid());
+    case 5: return fn(I5(), I2(), Mid());
+    default: return fn(I3(), IB(), Mid());
   }
   switch (stages) {
     case 2: return fn(I2(), IB(), One());

@@ -10,7 +10,8 @@ import cases
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [(20, 72, 72), (100, 72, 72), (20, 24, 16), (200, 40, 40)])
+@pytest.mark.parametrize("n", [(20, 72, 72), (100, 72, 72), (20, 24, 16), (200, 40, 40), (129, 40, 40),
+                               (192, 24, 30)])
 @pytest.mark.parametrize("periodic", [(1, 1, 1), (0, 0, 0)])
 @pytest.mark.parametrize("storage", ["fp32", "fp16", "bf16"])
 def test_any_number_of_stages(n, periodic, storage, monkeypatch):
