@@ -1175,8 +1175,19 @@ static cudaError_t with_shape(const Geom& g, int stages, int k, Fn fn) {
 // nodes, 16-bit storage beyond 1500) the direct kernel is faster in FP32
 // (900x100x90: 251 against 277 us) and slower in 16 bits (1400x80x70: 310
 // against 244), which takes three stages then.  0: the direct kernel.
+//
+// D2Q9 moves half the bytes a node of D3Q19 while a row costs the same hand-overs
+// between the warps: in FP32 the pipeline loses to the direct kernel at rows of
+// up to 600 nodes (600 x 2000: 20.8 and 19.7 us; 16 bits: 20.8 and 21.8), wins at
+// 900 (900 x 2000: 24.9 and 27.9) while the populations stay in the L2 cache and
+// loses beyond it (900 x 4000, 130 MB: 68.1 and 61.1; 1500 x 1500, 81 MB: 31.9 and
+// 33.9; 1500 x 2000, 108 MB: 54.1 and 48.5).
+constexpr long long LONG_2D_MAX_BYTES = 96ll << 20;
 template <class L, typename T>
 static int long_row_stages(const Geom& g, int sm_count) {
+  if (L::Q == 9 && sizeof(T) == 4 &&
+      (g.S[0] <= 750 || (long long)sizeof(T) * L::Q * g.Np > LONG_2D_MAX_BYTES))
+    return 0;
   // too few rows to keep the persistent blocks in turns (a 2-D channel of
   // 603 x 189 nodes takes 5 us either way)
   if ((long long)g.S[1] * g.S[2] < 8ll * sm_count) return 0;
